@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libdn_cuda.so")
 SOURCES = ["dn_capi.cu", "dn_config.cpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "--fmad=false", "-std=c++17",
+FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-split-compile=0", "-lineinfo", "--fmad=false", "-std=c++17",
          "-Xcompiler", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "include")]
 
 

@@ -30,6 +30,7 @@
 #include "dn_momentum.cuh"
 #include "dn_momentum_adjoint.cuh"
 #include "dn_multigrid.cuh"
+#include "dn_wpcg.cuh"
 
 using namespace dn;
 
@@ -590,6 +591,15 @@ struct dn_handle {
   int sw5_blocks_by_sw[kSweepWarpsPerCta + 1] = {};  // the same for each sweep-warp count up to sw5_budget
   size_t sw5_warp_smem[2] = {0, 0};  // per sweep warp, [constant operator, variable operator]
   int smem_optin = 0;
+  // pressure PCG in sweep order (dn_wpcg.cuh): the FP64 form, or the FP32 inner solves of the mixed form.
+  // sw = 0: not set up (no memory to spare, or a line too long for the shared hand-over lines)
+  struct WPlan {
+    int sw = 0, sw_budget = 0;                       // sweep warps per CTA, and the most that fit
+    int blocks_by_sw[kSweepWarpsPerCta + 1] = {};  // co-resident CTAs for each sweep-warp count
+    size_t warp_smem = 0;                            // shared bytes per sweep warp
+    void *mem = nullptr;                             // vectors and hand-over lines in sweep order
+    double *slots = nullptr;
+  } wp;
   double initial_mass = 0.0;
   long long launches = 0;
   std::string err;
@@ -602,8 +612,6 @@ struct dn_handle {
   float *fa5 = nullptr, *fl5 = nullptr, *fdinv5 = nullptr;
   float *fb = nullptr, *fx = nullptr, *fr = nullptr, *fz = nullptr, *fy = nullptr, *fp0 = nullptr, *fp1 = nullptr,
         *fap = nullptr;
-  int sw5f = 0, sw5f_blocks_max = 0;
-  size_t sw5f_warp_smem[2] = {0, 0};
   // mixed form, multigrid-preconditioned inner CG (dn_multigrid.cuh): the pressure hierarchy (level 0 = the
   // FP32 pressure operator fa5, with the inner CG's r / z and fy as its right-hand side / iterate / residual)
   // and the CH preconditioner's hierarchy (level 0 = the shifted Laplacian K + s I, own buffers).
@@ -969,6 +977,194 @@ enum StepSlot {
   kSPFactor = 21,  // the pressure factor's status (variable operator)
 };
 
+// ---- the pressure PCG in sweep order (dn_wpcg.cuh)
+// Vectors and lines of a grid, as consecutive pieces of one allocation.
+template <typename T>
+size_t wpcg_layout(int nx, int ny, bool px, bool var, char *base, WArgs<T> *P) {
+  size_t off = 0;
+  auto take = [&](size_t pairs) {
+    Pair<T> *q = reinterpret_cast<Pair<T> *>(base + off);
+    off += (pairs * sizeof(Pair<T>) + 255) & ~(size_t)255;
+    return q;
+  };
+  const size_t vp = w_vec_pairs(nx, ny), line = (size_t)w_line(ny);
+  WArgs<T> A{};
+  for (Pair<T> **v : {&A.r, &A.v, &A.z, &A.p0, &A.p1, &A.x, &A.ap, &A.q, &A.dg}) *v = take(vp);
+  if (var)
+    for (Pair<T> **v : {&A.aw, &A.as, &A.ga, &A.ha, &A.gn, &A.he}) *v = take(vp);
+  A.line_f = take((size_t)w_blocks(nx) * line);
+  A.line_b = take((size_t)w_blocks(nx) * line);
+  if (px) {
+    A.wrap_f = take(line);
+    A.wrap_b = take(line);
+  }
+  if (P) *P = A;
+  return off;
+}
+
+template <typename T>
+const void *wpcg_kernel(bool var, bool px, bool py) {
+  static const void *const k[8] = {
+      (const void *)k_wpcg<T, false, false, false>, (const void *)k_wpcg<T, false, false, true>,
+      (const void *)k_wpcg<T, false, true, false>,  (const void *)k_wpcg<T, false, true, true>,
+      (const void *)k_wpcg<T, true, false, false>,  (const void *)k_wpcg<T, true, false, true>,
+      (const void *)k_wpcg<T, true, true, false>,   (const void *)k_wpcg<T, true, true, true>};
+  return k[(var ? 4 : 0) + (px ? 2 : 0) + (py ? 1 : 0)];
+}
+
+// Sweep warps (blocks) per CTA: one.  Two on an SM slow each other down by more than the shorter hand-over inside a
+// CTA saves (192 x 384 split: 59.5 us of sweeps per iteration with one, 61.0 with two; 512 x 1024: 152 and 161); more
+// only where the CTAs would not fit the caller's share otherwise.
+template <typename T>
+int wpcg_sweep_warps(int nx, int ny, bool px, bool py, bool var, int optin, int cta_cap, int asked, size_t *warp_smem,
+                     int *budget) {
+  cudaFuncAttributes fa{};
+  if (cudaFuncGetAttributes(&fa, wpcg_kernel<T>(var, px, py)) != cudaSuccess) return 0;
+  if (!w_fits(nx, ny, px, py)) return 0;
+  const size_t per = w_warp_smem(var, ny, sizeof(T), px);
+  const size_t room = (size_t)optin > fa.sharedSizeBytes ? (size_t)optin - fa.sharedSizeBytes : 0;
+  const int nblk = w_blocks(nx);
+  // three warps for each block: its sweep warp, helper and stager
+  const int most = std::min((int)std::min<size_t>(kWBlock / 32 / 3, room / per), nblk);
+  *warp_smem = per;
+  *budget = most;
+  if (most < 1) return 0;
+  if (asked > 0) return std::min(asked, most);
+  int sw = 1;
+  while (sw < most && (nblk + sw - 1) / sw > cta_cap) ++sw;
+  return sw;
+}
+
+// CTAs of a solve: about rows_per_cta cells each, within the share and the co-resident limit; 0: not launchable
+int wpcg_blocks(long long n, long long rows_per_cta, int cta_cap, int nblk, int sw, int limit) {
+  const int sweep_ctas = (nblk + sw - 1) / sw;
+  int blocks = (int)std::min<long long>(cta_cap, (n + rows_per_cta - 1) / rows_per_cta);
+  blocks = std::min(std::max(std::max(1, blocks), sweep_ctas), std::min(limit, kMaxBlocks));
+  return blocks < sweep_ctas ? 0 : blocks;
+}
+
+template <typename T>
+void wpcg_problem(WArgs<T> &P, const Grid &G, bool var, int prec, int project, int max_it, double tol, double tol_abs) {
+  P.nx = G.nx;
+  P.ny = G.ny;
+  P.np = w_pairs(G.ny);
+  P.S = w_steps(G.ny);
+  P.nblk = w_blocks(G.nx);
+  P.px = G.px;
+  P.py = G.py;
+  P.prec = prec;
+  P.project = project;
+  P.max_it = max_it;
+  P.tol = tol;
+  P.tol_abs = tol_abs;
+  P.cx = (T)(-(1.0 / (G.dx * G.dx)));
+  P.cy = (T)(-(1.0 / (G.dy * G.dy)));
+  P.kappa = (T)((G.dy * G.dy) / (G.dx * G.dx));
+  P.scale = var ? (T)1 : -P.cy;
+}
+
+// The handle's plan: its buffers only while they take a small part of the free memory (the layout pads short
+// lines), so that a grid that filled the device before still fits.
+template <typename T>
+dn_status wpcg_setup(dn_handle *h) {
+  const dn_config &c = h->cfg;
+  const bool var = !use_split(c), px = c.periodic_x != 0, py = c.periodic_y != 0;
+  dn_handle::WPlan &W = h->wp;
+  const void *kern = wpcg_kernel<T>(var, px, py);
+  const int sw = wpcg_sweep_warps<T>(c.nx, c.ny, px, py, var, h->smem_optin, h->cta_cap, c.sweep_warps_per_cta,
+                                     &W.warp_smem, &W.sw_budget);
+  if (sw == 0) return DN_OK;
+  cudaFuncAttributes fa{};
+  DN_CUDA(h, cudaFuncGetAttributes(&fa, kern));
+  DN_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  h->smem_optin - (int)fa.sharedSizeBytes));
+  for (int w = 1; w <= W.sw_budget; ++w) {
+    int occ = 0;
+    DN_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWBlock, (size_t)w * W.warp_smem));
+    W.blocks_by_sw[w] = std::min(kMaxBlocks, occ * h->num_sms);
+  }
+  if (wpcg_blocks(h->n, h->rows_per_cta, h->cta_cap, w_blocks(c.nx), sw, W.blocks_by_sw[sw]) == 0) return DN_OK;
+  const size_t bytes = wpcg_layout<T>(c.nx, c.ny, px, var, nullptr, nullptr);
+  size_t free_b = 0, total_b = 0;
+  DN_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
+  if (bytes > free_b / 8) return DN_OK;
+  char *mem = nullptr;
+  DN_TRY(dalloc(h, &mem, bytes));
+  DN_TRY(dalloc(h, &W.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot));
+  W.mem = mem;
+  W.sw = sw;
+  return DN_OK;
+}
+
+// Prepares one solve on the handle's plan: arguments, launch shape, reduction slots and status word.
+template <typename T>
+dn_status wpcg_prepare(dn_handle *h, const T *b, T *x, const T *a5, const T *dinv, int prec, int project, int max_it,
+                       double tol, double tol_abs, WArgs<T> &P, int &blocks, size_t &smem) {
+  const dn_handle::WPlan &W = h->wp;
+  const bool var = !use_split(h->cfg);
+  wpcg_layout<T>(h->G.nx, h->G.ny, h->G.px != 0, var, static_cast<char *>(W.mem), &P);
+  wpcg_problem(P, h->G, var, prec, project, max_it, tol, tol_abs);
+  P.b = b;
+  P.x_out = x;
+  P.a5 = a5;
+  P.dinv = dinv;
+  P.slots = W.slots;
+  P.status = h->status;
+  P.out = h->scal + 8;
+  P.sw = W.sw;
+  P.warp_smem = (int)W.warp_smem;
+  P.prof = h->prof;
+  blocks = wpcg_blocks(h->n, h->rows_per_cta, h->cta_cap, P.nblk, W.sw, W.blocks_by_sw[W.sw]);
+  if (blocks == 0) return fail(h, DN_ERR_UNSUPPORTED, "not enough co-resident CTAs for the wavefront");
+  smem = (size_t)W.sw * W.warp_smem;
+  DN_CUDA(h, cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+  DN_CUDA(h, cudaMemsetAsync(W.slots, 0xff, (size_t)blocks * kWSlotSets * kWSlot * sizeof(double), h->stream));
+  return DN_OK;
+}
+
+// A persistent PCG kernel launched and, unless it is being recorded, its results read back: iterations and
+// residuals in out, its time added to phase_ms[slot], the 5-point kernels' split into pcg_split_ms.
+dn_status pcg_launch(dn_handle *h, const void *kern, int blocks, int threads, void **args, size_t smem, int slot,
+                     double out[4], double *rec) {
+  out[0] = out[1] = out[2] = out[3] = 0.0;
+  if (h->capturing) {
+    DN_CUDA(h, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, smem, h->stream));
+    h->launches++;
+    if (!rec) return DN_OK;  // status and results stay on the device (h->status, h->scal + 8)
+    k_rec_copy<<<1, 32, 0, h->stream>>>(h->scal + 8, 4, h->status, rec);
+    return check_launch(h, "k_rec_copy");
+  }
+  cudaEventRecord(h->kev[0], h->stream);
+  DN_CUDA(h, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, smem, h->stream));
+  cudaEventRecord(h->kev[1], h->stream);
+  h->launches++;
+  int st = 0;
+  DN_TRY(read_status(h, &st));
+  if (st != kDevOk) return dev_status_to_dn(h, st);
+  float ms = 0.0f;
+  cudaEventElapsedTime(&ms, h->kev[0], h->kev[1]);
+  h->phase_ms[slot] += ms;
+  double tmp[7];
+  DN_TRY(read_scalars(h, 7, tmp));
+  for (int k = 0; k < 4; ++k) out[k] = tmp[k];
+  if (slot == 4)  // the mixed form adds up its inner solves
+    for (int k = 0; k < 3; ++k)
+      h->pcg_split_ms[k] = (h->cfg.precision == DN_PRECISION_MIXED ? h->pcg_split_ms[k] : 0.0) + tmp[4 + k];
+  return DN_OK;
+}
+
+// The FP64 pressure PCG on the handle's compact b, x, a5, dinv5 (x holds zeros on entry).
+dn_status run_wpcg(dn_handle *h, int prec, int project, int max_it, double tol, double out[4], double *rec) {
+  WArgs<double> P{};
+  int blocks = 0;
+  size_t smem = 0;
+  DN_TRY(wpcg_prepare<double>(h, h->b, h->x, h->a5, h->dinv5, prec, project, max_it, tol, tol, P, blocks, smem));
+  P.mon = h->mon;
+  P.mon_cap = h->mon_cap;
+  void *args[] = {&P};
+  return pcg_launch(h, wpcg_kernel<double>(!use_split(h->cfg), h->G.px != 0, h->G.py != 0), blocks, kWBlock, args, smem, 4, out, rec);
+}
+
 // rec: where a solve recorded into a graph (h->capturing) leaves its out[0..4) and status (k_rec_copy);
 // nothing is read back then
 template <int S, int SWEEP>
@@ -980,42 +1176,24 @@ dn_status run_pcg(dn_handle *h, const double *a, const double *l, const double *
   DN_TRY((pcg_launch_args<S, SWEEP>(h, a, l, dinv, prec, project, max_it, tol, P, dyn_smem, blocks)));
   DN_TRY(reset_sync(h));
   void *args[] = {&P};
-  if (h->capturing) {
-    if (!rec) return fail(h, DN_ERR_UNSUPPORTED, "a recorded PCG solve needs a record");
-    DN_CUDA(h, cudaLaunchCooperativeKernel((const void *)k_pcg<S, SWEEP>, dim3(blocks), dim3(kBlock), args, dyn_smem,
-                                           h->stream));
-    h->launches++;
-    k_rec_copy<<<1, 32, 0, h->stream>>>(h->scal + 8, 4, h->status, rec);
-    out[0] = out[1] = out[2] = out[3] = 0.0;
-    return check_launch(h, "k_rec_copy");
-  }
-  cudaEventRecord(h->kev[0], h->stream);
-  DN_CUDA(h, cudaLaunchCooperativeKernel((const void *)k_pcg<S, SWEEP>, dim3(blocks), dim3(kBlock), args, dyn_smem,
-                                         h->stream));
-  cudaEventRecord(h->kev[1], h->stream);
-  h->launches++;
-  int st = 0;
-  DN_TRY(read_status(h, &st));
-  if (st != kDevOk) return dev_status_to_dn(h, st);
-  float ms = 0.0f;
-  cudaEventElapsedTime(&ms, h->kev[0], h->kev[1]);
-  h->phase_ms[S == 5 ? 4 : 5] += ms;
-  double tmp[7];
-  DN_TRY(read_scalars(h, 7, tmp));
-  for (int k = 0; k < 4; ++k) out[k] = tmp[k];
-  if (S == 5) {
-    h->pcg_split_ms[0] = tmp[4];
-    h->pcg_split_ms[1] = tmp[5];
-    h->pcg_split_ms[2] = tmp[6];
-  }
-  return DN_OK;
+  if (h->capturing && !rec) return fail(h, DN_ERR_UNSUPPORTED, "a recorded PCG solve needs a record");
+  return pcg_launch(h, (const void *)k_pcg<S, SWEEP>, blocks, kBlock, args, dyn_smem, S == 5 ? 4 : 5, out, rec);
 }
 
-// One FP32 inner PCG solve (the persistent kernel instantiated for float) on the handle's FP32 buffers.
+// One FP32 inner PCG solve (the persistent kernels instantiated for float) on the handle's FP32 buffers, from a
+// zero iterate.
 dn_status run_pcg32(dn_handle *h, int prec, int project, int max_it, double tol, double out[4]) {
+  const int its = std::max(1, max_it);
+  const double tol_abs = 0.0;  // an inner solve stops on its relative residual only
+  if (h->wp.sw > 0) {
+    WArgs<float> P{};
+    int blocks = 0;
+    size_t smem = 0;
+    DN_TRY(wpcg_prepare<float>(h, h->fb, h->fx, h->fa5, h->fdinv5, prec, project, its, tol, tol_abs, P, blocks, smem));
+    void *args[] = {&P};
+    return pcg_launch(h, wpcg_kernel<float>(!use_split(h->cfg), h->G.px != 0, h->G.py != 0), blocks, kWBlock, args, smem, 4, out, nullptr);
+  }
   PcgArgsT<float> P{};
-  P.mon = nullptr;
-  P.mon_cap = 0;
   P.A = SpOpT<float>{h->fa5, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py};
   P.l = h->fl5;
   P.dinv = h->fdinv5;
@@ -1029,9 +1207,9 @@ dn_status run_pcg32(dn_handle *h, int prec, int project, int max_it, double tol,
   P.p1 = h->fp1;
   P.ap = h->fap;
   P.project = project;
-  P.max_it = std::max(1, max_it);
+  P.max_it = its;
   P.tol = tol;
-  P.tol_abs = 0.0;  // an inner solve stops on its relative residual only
+  P.tol_abs = tol_abs;
   P.bar_count = h->bar_count;
   P.bar_gen = h->bar_gen;
   P.status = h->status;
@@ -1040,83 +1218,16 @@ dn_status run_pcg32(dn_handle *h, int prec, int project, int max_it, double tol,
   P.partials = h->partials;
   P.out = h->scal + 8;
   P.nsweep = h->nsweep;
-  P.warp_smem = 0;
-  size_t dyn_smem = 0;
-  // about 512 rows per CTA: the SpMV / update phases are latency-bound, so more CTAs shorten them
   const long long rows_per_cta = h->rows_per_cta;
   int blocks = (int)std::min<long long>(h->cta_cap,
                                         std::max<long long>(h->nsweep, (h->n + rows_per_cta - 1) / rows_per_cta));
   blocks = std::max(blocks, (h->nsweep + kBlock / 32 - 1) / (kBlock / 32));  // the wavefront warps' CTAs
   blocks = std::max(1, std::min(blocks, h->max_coop_blocks));
-  const bool staged = h->sw5f > 0;
-  if (staged) {
-    const bool var = !use_split(h->cfg);
-    Sweep5T<float> &W = P.s5;
-    W.nx = h->G.nx;
-    W.ny = h->G.ny;
-    W.n = (int)h->n;
-    W.px = h->G.px;
-    W.py = h->G.py;
-    W.prec = prec;
-    W.varcoef = var ? 1 : 0;
-    W.aW = h->fa5;
-    W.aS = h->fa5 + h->n;
-    W.aN = h->fa5 + 3 * h->n;
-    W.aE = h->fa5 + 4 * h->n;
-    W.cx = (float)(-(1.0 / (h->G.dx * h->G.dx)));
-    W.cy = (float)(-(1.0 / (h->G.dy * h->G.dy)));
-    W.dinv = h->fdinv5;
-    W.r = h->fr;
-    W.y = h->fy;
-    W.z = h->fz;
-    W.bnd_f = reinterpret_cast<float *>(h->bnd_f);  // the FP64 hand-over buffers, reused
-    W.bnd_b = reinterpret_cast<float *>(h->bnd_b);
-    W.wline0 = reinterpret_cast<float *>(h->wline0);
-    W.zlast = reinterpret_cast<float *>(h->zlast);
-    W.prog_f = h->prog;
-    W.prog_b = h->prog + kMaxBlocks * 8;
-    W.nsweep = h->nsweep5;
-    W.sw = h->sw5f;
-    W.status = h->status;
-    P.warp_smem = (int)h->sw5f_warp_smem[var ? 1 : 0];
-    W.warp_smem = P.warp_smem;
-    W.prof = h->prof;
-    dyn_smem = 64 + (size_t)h->sw5f * P.warp_smem;
-    const int sweep_ctas = (h->nsweep5 + h->sw5f - 1) / h->sw5f;
-    blocks = std::max(blocks, sweep_ctas);
-    blocks = std::min(blocks, h->sw5f_blocks_max);
-    if (blocks < sweep_ctas) return fail(h, DN_ERR_UNSUPPORTED, "not enough co-resident CTAs for the wavefront");
-  } else if ((long long)blocks * (kBlock / 32) < h->nsweep) {
+  if ((long long)blocks * (kBlock / 32) < h->nsweep)
     return fail(h, DN_ERR_UNSUPPORTED, "grid too wide for the co-resident wavefront warps");
-  }
   DN_TRY(reset_sync(h));
   void *args[] = {&P};
-  const void *kern = !staged ? (const void *)k_pcg<5, 0, float>
-                     : h->G.px ? (const void *)k_pcg<5, 4, float>
-                               : (const void *)k_pcg<5, 3, float>;
-  if (h->capturing) {  // recorded into a graph: status and results stay on the device (h->status, h->scal + 8)
-    DN_CUDA(h, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kBlock), args, dyn_smem, h->stream));
-    h->launches++;
-    out[0] = out[1] = out[2] = out[3] = 0.0;
-    return DN_OK;
-  }
-  cudaEventRecord(h->kev[0], h->stream);
-  DN_CUDA(h, cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kBlock), args, dyn_smem, h->stream));
-  cudaEventRecord(h->kev[1], h->stream);
-  h->launches++;
-  int st = 0;
-  DN_TRY(read_status(h, &st));
-  if (st != kDevOk) return dev_status_to_dn(h, st);
-  float ms = 0.0f;
-  cudaEventElapsedTime(&ms, h->kev[0], h->kev[1]);
-  h->phase_ms[4] += ms;
-  double tmp[7];
-  DN_TRY(read_scalars(h, 7, tmp));
-  for (int k = 0; k < 4; ++k) out[k] = tmp[k];
-  h->pcg_split_ms[0] += tmp[4];
-  h->pcg_split_ms[1] += tmp[5];
-  h->pcg_split_ms[2] += tmp[6];
-  return DN_OK;
+  return pcg_launch(h, (const void *)k_pcg<5, 0, float>, blocks, kBlock, args, 0, 4, out, nullptr);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -2814,6 +2925,9 @@ dn_status pressure_factor_solve(dn_handle *h, bool split, bool icc, dn_report *r
     DN_TRY(mixed_pressure(h, split, kind, out));
     rep->refinement_cycles = h->refinement_cycles;
     rep->mixed_inner_multigrid = h->mixed_used_mg ? 1 : 0;
+  } else if (h->wp.sw > 0) {
+    DN_TRY(run_wpcg(h, kind, h->has_dirichlet ? 0 : 1, cfg.poisson_iterations, cfg.pressure_tolerance, out,
+                    h->rec + kRecStep + kSP));
   } else if (h->sw5 > 0 && h->G.px) {
     DN_TRY((run_pcg<5, 4>(h, h->a5, h->l5, h->dinv5, kind, h->has_dirichlet ? 0 : 1, cfg.poisson_iterations,
                           cfg.pressure_tolerance, out, h->rec + kRecStep + kSP)));
@@ -3410,30 +3524,6 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
       A(mg_upload_chain(h, h->mgc));
       if (s != DN_OK) return bad(s, "device allocation failed: " + h->err);
     }
-    const int optin = h->smem_optin;
-    auto round16 = [](size_t b) { return (b + 15) & ~(size_t)15; };
-    const bool px = c.periodic_x != 0;
-    const bool stageable = !px || h->nsweep5 >= 2;
-    const void *k53f = px ? (const void *)k_pcg<5, 4, float> : (const void *)k_pcg<5, 3, float>;
-    h->sw5f_warp_smem[0] = round16(sweep_warp_smem(2, ny, 4, px));
-    h->sw5f_warp_smem[1] = round16(sweep_warp_smem(4, ny, 4, px));
-    const size_t per = h->sw5f_warp_smem[use_split(c) ? 0 : 1];
-    cudaFuncAttributes fa{};
-    cudaFuncGetAttributes(&fa, k53f);
-    const size_t budget = (size_t)optin > 64 + fa.sharedSizeBytes ? (size_t)optin - 64 - fa.sharedSizeBytes : 0;
-    int sw = stageable ? (int)std::min<size_t>(kSweepWarpsPerCta, budget / per) : 0;
-    sw = std::min(sw, h->nsweep5);
-    if (sw > 0 && c.sweep_warps_per_cta > 0) sw = std::min(sw, c.sweep_warps_per_cta);
-    h->sw5f = stageable ? sw : 0;
-    if (h->sw5f > 0) {
-      const size_t dyn = 64 + (size_t)sw * per;
-      cudaFuncSetAttribute(k53f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           std::max((int)dyn, optin - (int)fa.sharedSizeBytes));
-      int occf = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occf, k53f, kBlock, dyn);
-      h->sw5f_blocks_max = std::min(kMaxBlocks, std::max(0, occf) * h->num_sms);
-      if (h->sw5f_blocks_max == 0) h->sw5f = 0;
-    }
   }
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg<5, 0>, kBlock, 0);
@@ -3449,6 +3539,10 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
     occ = std::min(occ, occ4);
   }
   h->max_coop_blocks = std::min(kMaxBlocks, std::max(1, occ) * h->num_sms);
+  if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG) {
+    A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
+    if (s != DN_OK) return bad(s, "device allocation failed: " + h->err);
+  }
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bad(DN_ERR_CUDA, "initial synchronisation failed");
   *out = h;
   return DN_OK;
@@ -3783,15 +3877,20 @@ dn_status dn_autotune_pressure(dn_handle *h, int *rows_per_cta, int *sweep_warps
   const long long rows_c[] = {256, 512, 1024, 2048, 4096};
   // sweep-warp counts whose wavefront CTAs are co-resident; the FP64 staged path only (the mixed form's
   // FP32 wavefront keeps its own)
+  const bool fp64 = h->cfg.precision != DN_PRECISION_MIXED;
+  int &sw_now = fp64 && h->wp.sw > 0 ? h->wp.sw : h->sw5;
   std::vector<int> sws;
-  if (h->sw5 > 0 && h->cfg.precision != DN_PRECISION_MIXED) {
+  if (fp64 && h->wp.sw > 0) {
+    for (int w = 1; w <= h->wp.sw_budget; ++w)
+      if ((w_blocks(h->G.nx) + w - 1) / w <= h->wp.blocks_by_sw[w]) sws.push_back(w);
+  } else if (fp64 && h->sw5 > 0) {
     for (int w = 1; w <= h->sw5_budget; ++w)
       if ((h->nsweep5 + w - 1) / w <= h->sw5_blocks_by_sw[w]) sws.push_back(w);
   } else {
-    sws.push_back(h->sw5);
+    sws.push_back(sw_now);
   }
   const long long rows0 = h->rows_per_cta;
-  const int sw0 = h->sw5;
+  const int sw0 = sw_now;
   long long best_rows = rows0;
   int best_sw = sw0;
   double best = INFINITY;
@@ -3803,7 +3902,7 @@ dn_status dn_autotune_pressure(dn_handle *h, int *rows_per_cta, int *sweep_warps
     for (long long rows : rows_c)
       for (int sw : sws) {
         h->rows_per_cta = rows;
-        h->sw5 = sw;
+        sw_now = sw;
         ++h->graph_epoch;  // recorded solves hold launch shapes
         dn_report rep{};
         cudaEventRecord(e0, h->stream);
@@ -3822,7 +3921,7 @@ dn_status dn_autotune_pressure(dn_handle *h, int *rows_per_cta, int *sweep_warps
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   h->rows_per_cta = st == DN_OK ? best_rows : rows0;
-  h->sw5 = st == DN_OK ? best_sw : sw0;
+  sw_now = st == DN_OK ? best_sw : sw0;
   ++h->graph_epoch;
   if (st != DN_OK) return st;
   if (rows_per_cta) *rows_per_cta = (int)best_rows;
@@ -4660,7 +4759,10 @@ dn_status static_fail(char *err, size_t err_len, dn_status s, const char *fmt, .
 // Byte offsets of the sub-buffers inside the scratch array, each on a 256-byte boundary.
 struct StaticLayout {
   size_t bar_count, bar_gen, status, prog, partials, scal, prof;
-  size_t b, x, r, z, y, p0, p1, ap, a5, l5, d5, dinv5, pe, bnd_f, bnd_b, wline0, zlast;
+  size_t b, x, a5, dinv5, pe;
+  // from `tail` on: the factor's work arrays, dead once dinv5 is made, and the vectors of the PCG on compact
+  // rows; the PCG in sweep order lays its own over the same bytes
+  size_t tail, l5, d5, r, z, y, p0, p1, ap, bnd_f, bnd_b, wline0, zlast;
   size_t total;
 };
 
@@ -4681,12 +4783,15 @@ StaticLayout static_layout(int nx, int ny, int g) {
   L.partials = take(2 * (size_t)kMaxBlocks * 8 * sizeof(double));
   L.scal = take(64 * sizeof(double));
   L.prof = take(64 * sizeof(double));
-  for (size_t *v : {&L.b, &L.x, &L.r, &L.z, &L.y, &L.p0, &L.p1, &L.ap}) *v = take(n * sizeof(double));
+  L.b = take(n * sizeof(double));
+  L.x = take(n * sizeof(double));
   L.a5 = take(5 * n * sizeof(double));
-  L.l5 = take(5 * n * sizeof(double));
-  L.d5 = take(n * sizeof(double));
   L.dinv5 = take(n * sizeof(double));
   L.pe = take((size_t)(nx + 2 * g) * (ny + 2 * g) * sizeof(double));
+  L.tail = off;
+  L.l5 = take(5 * n * sizeof(double));
+  L.d5 = take(n * sizeof(double));
+  for (size_t *v : {&L.r, &L.z, &L.y, &L.p0, &L.p1, &L.ap}) *v = take(n * sizeof(double));
   L.bnd_f = take(2 * nsweep * ny * sizeof(double));
   L.bnd_b = take(2 * nsweep * ny * sizeof(double));
   L.wline0 = take(2 * (size_t)ny * sizeof(double));
@@ -4896,6 +5001,47 @@ dn_status dn_pressure_solve_static(const dn_config *cfg, int step, const double 
   // the persistent PCG kernel, launched with the default shape a handle would use for this grid and
   // configuration (device_share included); shapes a handle picked with dn_autotune_pressure are not known
   // here and are not reproduced (pass them as pcg_rows_per_cta / sweep_warps_per_cta)
+  const long long rows_per_cta = c.pcg_rows_per_cta > 0 ? c.pcg_rows_per_cta : kPcgRowsPerCta;
+  const int cta_cap = std::max(1, D.num_sms / std::max(1, c.device_share));
+  // in sweep order (dn_wpcg.cuh) when its padded vectors fit the scratch array beside the operator
+  bool solved = false;
+  {
+    const bool var = !split;
+    const void *kern = wpcg_kernel<double>(var, G.px != 0, G.py != 0);
+    WArgs<double> Q{};
+    int budget = 0, occ = 0;
+    size_t per = 0;
+    const int wsw = wpcg_sweep_warps<double>(nx, ny, G.px != 0, G.py != 0, var, D.smem_optin, cta_cap, c.sweep_warps_per_cta,
+                                             &per, &budget);
+    if (wsw > 0) {
+      cudaFuncAttributes fa{};
+      DN_SCUDA(cudaFuncGetAttributes(&fa, kern));
+      DN_SCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    D.smem_optin - (int)fa.sharedSizeBytes));
+      DN_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kWBlock, (size_t)wsw * per));
+    }
+    const int blocks = wsw > 0 ? wpcg_blocks(n, rows_per_cta, cta_cap, w_blocks(nx), wsw,
+                                             std::min(kMaxBlocks, occ * D.num_sms))
+                               : 0;
+    const size_t vec_bytes = wpcg_layout<double>(nx, ny, G.px != 0, var, base + L.tail, &Q);
+    const size_t slot_bytes = (size_t)blocks * kWSlotSets * kWSlot * sizeof(double);
+    if (blocks > 0 && L.tail + vec_bytes + slot_bytes <= (size_t)DN_STATIC_SCRATCH_BYTES) {
+      wpcg_problem(Q, G, var, kind, has_dirichlet ? 0 : 1, c.poisson_iterations, c.pressure_tolerance, c.pressure_tolerance);
+      Q.b = b;
+      Q.x_out = x;
+      Q.a5 = a5;
+      Q.dinv = dptr(L.dinv5);
+      Q.slots = dptr(L.tail + vec_bytes);
+      Q.status = status;
+      Q.out = scal + 8;
+      Q.sw = wsw;
+      Q.warp_smem = (int)per;
+      DN_SCUDA(cudaMemsetAsync(Q.slots, 0xff, slot_bytes, st));
+      void *qargs[] = {&Q};
+      DN_SCUDA(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kWBlock), qargs, (size_t)wsw * per, st));
+      solved = true;
+    }
+  }
   PcgArgs P{};
   P.A = A;
   P.l = dptr(L.l5);
@@ -4922,8 +5068,6 @@ dn_status dn_pressure_solve_static(const dn_config *cfg, int step, const double 
   P.out = scal + 8;
   P.nsweep = nsweep;
   P.warp_smem = 0;
-  const long long rows_per_cta = c.pcg_rows_per_cta > 0 ? c.pcg_rows_per_cta : kPcgRowsPerCta;
-  const int cta_cap = std::max(1, D.num_sms / std::max(1, c.device_share));
   int blocks = (int)std::min<long long>(cta_cap, std::max<long long>(nsweep, (n + rows_per_cta - 1) / rows_per_cta));
   blocks = std::max(blocks, (nsweep + kBlock / 32 - 1) / (kBlock / 32));  // the wavefront warps' CTAs
   blocks = std::max(1, std::min(blocks, D.max_coop_blocks));
@@ -4931,7 +5075,7 @@ dn_status dn_pressure_solve_static(const dn_config *cfg, int step, const double 
   int sw = 0, sw_blocks_max = 0;
   size_t warp_smem = 0;
   const void *k53 = G.px ? (const void *)k_pcg<5, 4> : (const void *)k_pcg<5, 3>;
-  if (!G.px || nsweep5 >= 2) {
+  if (!solved && (!G.px || nsweep5 >= 2)) {
     const size_t per = (sweep_warp_smem(split ? 2 : 4, ny, 8, G.px != 0) + 15) & ~(size_t)15;
     const size_t budget = (size_t)D.smem_optin > 64 + 2304 ? (size_t)D.smem_optin - 64 - 2304 : 0;
     sw = (int)std::min<size_t>(kSweepWarpsPerCta, budget / per);
@@ -4955,7 +5099,8 @@ dn_status dn_pressure_solve_static(const dn_config *cfg, int step, const double 
     }
   }
   void *args[] = {&P};
-  if (sw > 0) {
+  if (solved) {
+  } else if (sw > 0) {
     Sweep5 &W = P.s5;
     W.nx = nx;
     W.ny = ny;
