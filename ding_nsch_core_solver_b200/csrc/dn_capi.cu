@@ -30,6 +30,7 @@
 #include "dn_momentum.cuh"
 #include "dn_momentum_adjoint.cuh"
 #include "dn_multigrid.cuh"
+#include "dn_wch.cuh"
 #include "dn_wpcg.cuh"
 
 using namespace dn;
@@ -600,6 +601,12 @@ struct dn_handle {
     void *mem = nullptr;                             // vectors and hand-over lines in sweep order
     double *slots = nullptr;
   } wp;
+  // Cahn-Hilliard PCG swept by many CTAs (dn_wch.cuh); blocks = 0: not set up (periodic y, the mixed form, or no
+  // memory to spare)
+  struct CPlan {
+    int blocks = 0;  // co-resident CTAs
+    CArgs args{};    // coefficients and lines
+  } cp;
   double initial_mass = 0.0;
   long long launches = 0;
   std::string err;
@@ -1163,6 +1170,75 @@ dn_status run_wpcg(dn_handle *h, int prec, int project, int max_it, double tol, 
   P.mon_cap = h->mon_cap;
   void *args[] = {&P};
   return pcg_launch(h, wpcg_kernel<double>(!use_split(h->cfg), h->G.px != 0, h->G.py != 0), blocks, kWBlock, args, smem, 4, out, rec);
+}
+
+// ---- the Cahn-Hilliard PCG swept by many CTAs (dn_wch.cuh)
+dn_status wch_setup(dn_handle *h) {
+  const dn_config &c = h->cfg;
+  dn_handle::CPlan &W = h->cp;
+  if (!c_fits(c.nx, c.periodic_x != 0, c.periodic_y != 0) || c_smem() + 4096 > (size_t)h->smem_optin) return DN_OK;
+  DN_CUDA(h, cudaFuncSetAttribute(k_wch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c_smem()));
+  int occ = 0;
+  DN_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wch, kBlock, c_smem()));
+  const int limit = std::min(kMaxBlocks, occ * h->num_sms), nblk = w_blocks(c.nx);
+  if (nblk > limit) return DN_OK;
+  const size_t vp = c_vec_pairs(c.nx, c.ny), line = (size_t)c_line(c.ny), np = (size_t)w_pairs(c.ny);
+  const size_t pairs = 13 * vp + 4 * (size_t)nblk * line + (c.periodic_x ? 4 * line + 10 * np : 0);
+  size_t free_b = 0, total_b = 0;
+  DN_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
+  if (pairs * sizeof(Pair<double>) > free_b / 8) return DN_OK;
+  Pair<double> *m = nullptr;
+  DN_TRY(dalloc(h, &m, pairs));
+  CArgs &A = W.args;
+  DN_TRY(dalloc(h, &A.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot));
+  auto take = [&](size_t k) {
+    Pair<double> *q = m;
+    m += k;
+    return q;
+  };
+  A.np = (int)np;
+  A.S = c_steps(c.ny);
+  A.nblk = nblk;
+  A.v = take(vp);
+  for (int t = 0; t < 6; ++t) {
+    A.f[t] = take(vp);
+    A.u[t] = take(vp);
+  }
+  for (int d = 0; d < 2; ++d) A.line[d] = take(2 * (size_t)nblk * line);
+  if (c.periodic_x) {
+    for (int d = 0; d < 2; ++d) A.wrap[d] = take(2 * line);
+    for (int t = 0; t < 5; ++t) {
+      A.wf[t] = take(np);
+      A.wu[t] = take(np);
+    }
+  }
+  W.blocks = limit;
+  return DN_OK;
+}
+
+dn_status run_wch(dn_handle *h, double out[4], double *rec) {
+  CArgs C = h->cp.args;
+  PcgArgs &P = C.P;
+  P.A = SpOp{h->a13, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py};
+  P.prec = kPrecLDLT;
+  P.b = h->b;
+  P.x = h->x;
+  P.r = h->r;
+  P.z = h->z;
+  P.p0 = h->p0;
+  P.p1 = h->p1;
+  P.ap = h->ap;
+  P.max_it = h->cfg.ch_inner_iterations;
+  P.tol = P.tol_abs = h->cfg.ch_tolerance;
+  P.status = h->status;
+  P.out = h->scal + 8;
+  C.dinv = h->dinv13;
+  const int blocks = wpcg_blocks(h->n, h->rows_per_cta, h->cta_cap, C.nblk, 1, h->cp.blocks);
+  DN_CUDA(h, cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
+  DN_CUDA(h, cudaMemsetAsync(C.slots, 0xff, (size_t)blocks * kWSlotSets * kWSlot * sizeof(double), h->stream));
+  if (h->capturing && !rec) return fail(h, DN_ERR_UNSUPPORTED, "a recorded PCG solve needs a record");
+  void *args[] = {&C};
+  return pcg_launch(h, (const void *)k_wch, blocks, kBlock, args, c_smem(), 5, out, rec);
 }
 
 // rec: where a solve recorded into a graph (h->capturing) leaves its out[0..4) and status (k_rec_copy);
@@ -2046,7 +2122,11 @@ dn_status ensure_ch_system(dn_handle *h, double alpha0) {
     DN_TRY(check_launch(h, "k_diag_inverse"));
   } else {
     h->ch_prec = kPrecLDLT;
-    if (h->rows13.lval != nullptr) {
+    if (h->cp.blocks > 0) {
+      k_wch_setup<<<blocks_for((long long)c_vec_pairs(h->G.nx, h->G.ny)), 256, 0, h->stream>>>(
+          SpOp{h->a13, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F, h->cp.args);
+      DN_TRY(check_launch(h, "k_wch_setup"));
+    } else if (h->rows13.lval != nullptr) {
       k_rows13<<<blocks_for(h->n), 256, 0, h->stream>>>(SpOp{h->a13, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F,
                                                        h->rows13);
       DN_TRY(check_launch(h, "k_rows13"));
@@ -2054,6 +2134,13 @@ dn_status ensure_ch_system(dn_handle *h, double alpha0) {
   }
   h->ch_alpha0 = alpha0;
   return DN_OK;
+}
+
+// The ILDLT-preconditioned CG: swept by many CTAs, or (periodic y) by one.
+dn_status run_ch_ldlt(dn_handle *h, double out[4], double *rec) {
+  if (h->cp.blocks > 0) return run_wch(h, out, rec);
+  return run_pcg<13, 1>(h, h->a13, h->l13, h->dinv13, kPrecLDLT, 0, h->cfg.ch_inner_iterations, h->cfg.ch_tolerance, out,
+                        rec);
 }
 
 // solve_phase_linear_system_eq25, phase_field.cpp:437-503; b = rhs, x = initial guess (compact).  On exit x
@@ -2069,8 +2156,7 @@ dn_status ch_linear_solve(dn_handle *h, double alpha0, dn_report *rep, double *i
     // (phase_field.cpp:468-473) in a conditional branch
     double *R = h->rec + kRecStep;
     if (h->ch_prec == kPrecLDLT) {
-      DN_TRY((run_pcg<13, 1>(h, h->a13, h->l13, h->dinv13, kPrecLDLT, 0, h->cfg.ch_inner_iterations,
-                             h->cfg.ch_tolerance, out, R + kSChPcg)));
+      DN_TRY(run_ch_ldlt(h, out, R + kSChPcg));
       cudaGraphConditionalHandle retry = 0;
       DN_TRY(cond_create(h, &retry));
       k_cond_breakdown<<<1, 32, 0, h->stream>>>(h->status, retry);
@@ -2093,8 +2179,7 @@ dn_status ch_linear_solve(dn_handle *h, double alpha0, dn_report *rep, double *i
   } else if (!mixed_done) {
     dn_status s;
     if (h->ch_prec == kPrecLDLT)
-      s = run_pcg<13, 1>(h, h->a13, h->l13, h->dinv13, kPrecLDLT, 0, h->cfg.ch_inner_iterations, h->cfg.ch_tolerance,
-                         out);
+      s = run_ch_ldlt(h, out, nullptr);
     else
       s = run_pcg<13, 2>(h, h->a13, h->l13, h->dinv13, kPrecDiag, 0, h->cfg.ch_inner_iterations, h->cfg.ch_tolerance,
                          out);
@@ -3539,6 +3624,7 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
     occ = std::min(occ, occ4);
   }
   h->max_coop_blocks = std::min(kMaxBlocks, std::max(1, occ) * h->num_sms);
+  if (c.precision != DN_PRECISION_MIXED && solve_ch(c)) A(wch_setup(h));
   if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG) {
     A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
     if (s != DN_OK) return bad(s, "device allocation failed: " + h->err);
