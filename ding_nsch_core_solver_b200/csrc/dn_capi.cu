@@ -1375,6 +1375,7 @@ dn_status mg_alloc(dn_handle *h, MgHier &H, int nx, int ny, const BCSide *sides)
   H.fold.py = h->G.py;
   cudaFuncSetAttribute(k_mg_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)(sizeof(double) * kMgCoarseMax * kMgCoarseMax));
+  cudaFuncSetAttribute(k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMgBottomSmem);
   return DN_OK;
 }
 
@@ -1415,23 +1416,19 @@ dn_status mg_setup(dn_handle *h, MgHier &H, bool *usable) {
 // x0 = B b0: one V-cycle from level 0 with right-hand side b0 and result x0 (level 0's residual buffer is
 // H.lv[0].r)
 dn_status mg_vcycle_launch(dn_handle *h, MgHier &H, float *b0, float *x0) {
-  const int L = H.levels(), px = h->G.px, py = h->G.py;
+  const int L = H.levels();
   H.lv[0].b = b0;
   H.lv[0].x = x0;
-  // levels from `bottom` down run inside one CTA (k_mg_bottom); the ones above get a launch per phase
+  // the levels of at most kMgSmemCells cells run inside one CTA (k_mg_bottom), the ones above as one launch per
+  // level and direction
   int bottom = L - 1;
-  while (bottom > 0 && (long long)H.lv[bottom - 1].nx * H.lv[bottom - 1].ny <= kMgBottomCells) --bottom;
-  auto smooth = [&](const MgLevel &M, int color, int first) -> dn_status {
-    return launch_pdl(h, "k_mg_smooth", k_mg_smooth, dim3(blocks_for((long long)M.nx * (M.ny / 2))), dim3(256), 0, M, color, first, px, py);
+  while (bottom > 0 && (long long)H.lv[bottom - 1].nx * H.lv[bottom - 1].ny <= kMgSmemCells) --bottom;
+  auto tiles = [](const MgLevel &M, int rows, int cols) {
+    return dim3((unsigned)((M.ny + cols - 1) / cols), (unsigned)((M.nx + rows - 1) / rows));
   };
   for (int l = 0; l < bottom; ++l) {
     const MgLevel F = mg_level(H, l), C = mg_level(H, l + 1);
-    for (int k = 0; k < kMgSweeps; ++k) {
-      DN_TRY(smooth(F, 0, k == 0));
-      DN_TRY(smooth(F, 1, 0));
-    }
-    DN_TRY(launch_pdl(h, "k_mg_residual", k_mg_residual, dim3(blocks_for((long long)F.nx * F.ny)), dim3(256), 0, F, px, py));
-    DN_TRY(launch_pdl(h, "k_mg_restrict", k_mg_restrict, dim3(blocks_for((long long)C.nx * C.ny)), dim3(256), 0, F, C, H.fold));
+    DN_TRY(launch_pdl(h, "k_mg_down", k_mg_down, tiles(F, kMgDownRows, kMgDownCols), dim3(kMgTileThreads), 0, F, C, H.fold));
   }
   MgChain ch{};
   for (int l = 0; l < L; ++l) ch.lv[l] = mg_level(H, l);
@@ -1439,19 +1436,15 @@ dn_status mg_vcycle_launch(dn_handle *h, MgHier &H, float *b0, float *x0) {
   ch.last = L - 1;
   ch.fold = H.fold;
   ch.inv = H.inv;
-  DN_TRY(launch_pdl(h, "k_mg_bottom", k_mg_bottom, dim3(1), dim3(1024), 0, ch));
+  DN_TRY(launch_pdl(h, "k_mg_bottom", k_mg_bottom, dim3(1), dim3(kMgBottomThreads), kMgBottomSmem, ch));
   for (int l = bottom - 1; l >= 0; --l) {
     const MgLevel F = mg_level(H, l), C = mg_level(H, l + 1);
-    DN_TRY(launch_pdl(h, "k_mg_prolong", k_mg_prolong, dim3(blocks_for((long long)F.nx * F.ny)), dim3(256), 0, C, F, H.fold));
-    for (int k = 0; k < kMgSweeps; ++k) {
-      DN_TRY(smooth(F, 1, 0));
-      DN_TRY(smooth(F, 0, 0));
-    }
+    DN_TRY(launch_pdl(h, "k_mg_up", k_mg_up, tiles(F, kMgUpRows, kMgUpCols), dim3(kMgTileThreads), 0, C, F, H.fold));
   }
   return DN_OK;
 }
 
-// The V-cycle's ~11 launches per level are replayed from a CUDA graph captured on first use for this
+// The V-cycle's launches are replayed from a CUDA graph captured on first use for this
 // (hierarchy, b0, x0): the kernels' arguments are the level buffers' pointers, which never change, and the
 // operators are rewritten in place by mg_setup.
 dn_status mg_vcycle(dn_handle *h, MgHier &H, float *b0, float *x0) {

@@ -27,6 +27,8 @@
 
 #include <cooperative_groups.h>
 
+#include <type_traits>
+
 #include "dn_common.cuh"
 #include "dn_krylov.cuh"
 
@@ -49,44 +51,6 @@ struct MgFold {
   float s[4];
   int px, py;
 };
-
-__device__ __forceinline__ float mg_row_sum(const MgLevel &L, const float *x, int i, int j, long long r, long long n,
-                                            int px, int py) {
-  // sum of the off-diagonal terms a_s * x_nb, FP32 accumulation in slot order
-  float s = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    if (k == 2) continue;
-    const float a = L.a[(size_t)k * n + r];
-    if (a != 0.0f) {
-      const long long c = slot_col<5>(i, j, k, L.nx, L.ny, px, py);
-      if (c >= 0) s += a * x[c];
-    }
-  }
-  return s;
-}
-
-// Red-black Gauss-Seidel half sweep at cell t of the colour's cells ((i + j) & 1 == color); ny is even on every
-// smoothed level, so each row holds ny/2 cells of each colour.  first: the iterate is zero on entry, so the
-// colour's cells take b / diag and the other colour's cells are set to zero.
-__device__ __forceinline__ void mg_smooth_at(const MgLevel &L, int color, int first, int px, int py, unsigned t) {
-  const int half = L.ny >> 1;
-  const int i = (int)(t / (unsigned)half);
-  const int j = 2 * (int)(t - (unsigned)i * (unsigned)half) + ((i + color) & 1);
-  const long long n = (long long)L.nx * L.ny;
-  const long long r = (long long)i * L.ny + j;
-  float s = L.b[r];
-  if (!first) s -= mg_row_sum(L, L.x, i, j, r, n, px, py);
-  L.x[r] = s / L.a[2 * n + r];
-  if (first) L.x[(long long)i * L.ny + (j ^ 1)] = 0.0f;
-}
-
-// r = b - A x at cell t
-__device__ __forceinline__ void mg_residual_at(const MgLevel &L, int px, int py, unsigned t) {
-  const unsigned n = (unsigned)L.nx * (unsigned)L.ny;
-  const int i = (int)(t / (unsigned)L.ny), j = (int)(t - (unsigned)i * (unsigned)L.ny);
-  L.r[t] = L.b[t] - (L.a[2 * (size_t)n + t] * L.x[t] + mg_row_sum(L, L.x, i, j, t, n, px, py));
-}
 
 // 1D bilinear weight of coarse index I in the interpolation of fine index i (fine extent 2 * nc)
 __device__ __forceinline__ float mg_w1(int i, int I, int nc, int per, float s_lo, float s_hi) {
@@ -172,78 +136,498 @@ __device__ __forceinline__ void mg_prolong_at(const MgLevel &C, const MgLevel &F
   F.x[t] += v;
 }
 
-// one launch per phase on the levels above kMgBottomCells cells
-__global__ void k_mg_smooth(MgLevel L, int color, int first, int px, int py) {
-  pdl_entry();
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (unsigned)L.nx * (unsigned)(L.ny >> 1)) mg_smooth_at(L, color, first, px, py, t);
+// ---------------------------------------------------------------------------------------------------
+// The V-cycle of the large grids: one launch per level and direction.
+//
+// A half sweep does two operations per operator value it reads, so a level is bound by reading its operator
+// (five values per cell) as often as it is swept: nine times per V-cycle when every phase is a launch, plus
+// the launches themselves, which on the coarser levels are all of the time.  Here a CTA owns a tile of the
+// level, reads the operator of the tile and of a halo around it once into registers, and runs all of a
+// direction's phases on it: k_mg_down the four half sweeps before the coarse correction, the residual and its
+// restriction, k_mg_up the prolongation and the four half sweeps after it.  A phase is wrong in one more ring
+// of the region's cells than the phase before (they miss a neighbour), so the halo is as wide as the phases
+// are many, and what the tile's own cells hold is what phase-by-phase sweeps of the whole level leave there,
+// bit for bit: every cell is updated from the same values in the same order.
+//
+// A region is kMgRegionRows x kMgRegionCols cells: a lane holds a pair of columns (one cell of each colour), a warp
+// kMgRows rows.  Which cell of a pair has the phase's colour depends only on the row, so the choice is made
+// at compile time; a row's left and right neighbours come by shuffle, the rows above and below from the same
+// thread's registers or, at a warp's edge, through shared memory (one barrier per phase).  Cells outside a
+// walled grid get a zero row and stay zero; across a periodic side the region holds copies of the cells of
+// the other side.  The swept iterate goes to the level's residual buffer on the way down (no residual is
+// stored) and to x on the way up, so no CTA overwrites what another still reads as its halo.
+//
+// The operator is loaded before griddepcontrol.wait: no kernel of a V-cycle, nor the one launched before it,
+// writes an operator.
+//
+// 32 x 64 regions with three CTAs of eight warps per SM cover 1.9 (down) and 1.5 (up) times the cells, but where
+// 64 x 64 ones (1.5 and 1.3 times; one CTA of 16 warps by their registers) load, wait and sweep in turn, they
+// overlap.  Measured, us per launch in a chain of launches, 32 x 64 / 64 x 64: level of 2M cells down 29.5 / 34.7,
+// up 26.3 / 31.7; of 512K cells 11.2 / 11.8 and 7.8 / 12.3; of at most 100K cells, where a launch is latency,
+// 4.8 / 5.8 and 5.1 / 6.1.  A V-cycle of 11 launches per level and a bottom of 8192 cells in global memory took 373 us
+// at 1024 x 2048 and 139 us at 192 x 384 cells; this form takes 129 and 41.
+// ---------------------------------------------------------------------------------------------------
+constexpr int kMgRegionRows = 32, kMgRegionCols = 64;
+constexpr int kMgRows = 4;                        // rows of the region per warp (even)
+constexpr int kMgWarps = kMgRegionRows / kMgRows;
+constexpr int kMgTileThreads = 32 * kMgWarps;
+// halo before the tile's first row / column: one ring per phase (half sweeps, residual, restriction), and the
+// region's first column is even, so that pairs are aligned; the tile is even in both directions
+constexpr int kMgDownRow = 2 * kMgSweeps + 1, kMgDownCol = (kMgDownRow + 1) & ~1;
+constexpr int kMgDownRows = kMgRegionRows - 2 * kMgDownRow, kMgDownCols = (kMgRegionCols - kMgDownCol - kMgDownRow) & ~1;
+constexpr int kMgUp = 2 * kMgSweeps, kMgUpCols = kMgRegionCols - 2 * kMgUp, kMgUpRows = kMgRegionRows - 2 * kMgUp;
+static_assert(kMgRows % 2 == 0 && kMgDownRows % 2 == 0 && kMgUp % 2 == 0, "coarse cells and pairs are not cut");
+
+// The weights of fine cells 2 I - 1 .. 2 I + 2 in coarse cell I of nc >= 2: mg_w1's values, without its branches
+__device__ __forceinline__ void mg_w4(int I, int nc, int per, float s_lo, float s_hi, float (&w)[4]) {
+  const bool lo = !per && I == 0, hi = !per && I == nc - 1;
+  w[0] = lo ? 0.0f : 0.25f;
+  w[1] = lo ? 0.75f + 0.25f * s_lo : 0.75f;
+  w[2] = hi ? 0.75f + 0.25f * s_hi : 0.75f;
+  w[3] = hi ? 0.0f : 0.25f;
 }
-__global__ void k_mg_residual(MgLevel L, int px, int py) {
-  pdl_entry();
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (unsigned)L.nx * (unsigned)L.ny) mg_residual_at(L, px, py, t);
+// sum of w_i w_j r(i, j) over the 4 x 4 fine cells of a coarse cell, a row at a time (a cell outside has weight
+// zero and r = 0 or a cell's value)
+template <class R>
+__device__ __forceinline__ float mg_restrict_sum(const float (&wx)[4], const float (&wy)[4], R &&r) {
+  float sum = 0.0f;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    float row = 0.0f;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) row += wy[b] * r(a, b);
+    sum += wx[a] * row;
+  }
+  return sum;
 }
-__global__ void k_mg_restrict(MgLevel F, MgLevel C, MgFold fold) {
-  pdl_entry();
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (unsigned)C.nx * (unsigned)C.ny) mg_restrict_at(F, C, fold, t);
-}
-__global__ void k_mg_prolong(MgLevel C, MgLevel F, MgFold fold) {
-  pdl_entry();
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (unsigned)F.nx * (unsigned)F.ny) mg_prolong_at(C, F, fold, t);
+// index k of an extent of n cells, which may lie outside it: wrapped when periodic, else -1
+__device__ __forceinline__ int mg_wrap(int k, int n, int per) {
+  if (k >= 0 && k < n) return k;
+  if (!per) return -1;
+  k %= n;
+  return k < 0 ? k + n : k;
 }
 
-// The bottom of the V-cycle in one CTA: levels first .. last-1 (each at most kMgBottomCells cells) smoothed,
-// restricted, the coarsest (last) solved with its inverse, then prolonged and smoothed back up to `first`.
-// Phases are separated by __syncthreads instead of kernel boundaries; every cell sees the same operations
-// in the same order as with the per-phase kernels, so the result is the same.
+// A thread's part of a region: kMgRows rows of a pair of columns
+struct MgTile {
+  float a[kMgRows][4][2], d[kMgRows][2], b[kMgRows][2], x[kMgRows][2];  // a: W, S, N, E
+  int row[kMgRows];  // the level's row, -1 outside
+  int col;           // the pair's first column, -1 outside
+  unsigned lane, warp;
+};
+
+// the rows and columns of the region whose first cell is (i0, j0), and its operator
+__device__ __forceinline__ void mg_tile_operator(MgTile &T, const MgLevel &L, int i0, int j0, int px, int py) {
+  T.lane = threadIdx.x & 31u;
+  T.warp = threadIdx.x >> 5;
+  T.col = mg_wrap(j0 + 2 * (int)T.lane, L.ny, py);
+  const size_t n = (size_t)L.nx * L.ny;
+#pragma unroll
+  for (int q = 0; q < kMgRows; ++q) {
+    T.row[q] = mg_wrap(i0 + (int)T.warp * kMgRows + q, L.nx, px);
+    const bool in = T.row[q] >= 0 && T.col >= 0;
+    const size_t r = in ? (size_t)T.row[q] * L.ny + T.col : 0;
+    constexpr int ks[4] = {0, 1, 3, 4};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 v = in ? __ldg((const float2 *)(L.a + ks[k] * n + r)) : make_float2(0.0f, 0.0f);
+      T.a[q][k][0] = v.x;
+      T.a[q][k][1] = v.y;
+    }
+    const float2 v = in ? __ldg((const float2 *)(L.a + 2 * n + r)) : make_float2(1.0f, 1.0f);
+    T.d[q][0] = v.x;
+    T.d[q][1] = v.y;
+  }
+}
+__device__ __forceinline__ void mg_tile_load(const MgTile &T, const float *g, int ny, float (&v)[kMgRows][2]) {
+#pragma unroll
+  for (int q = 0; q < kMgRows; ++q) {
+    float2 w = make_float2(0.0f, 0.0f);
+    if (T.row[q] >= 0 && T.col >= 0) w = *(const float2 *)(g + (size_t)T.row[q] * ny + T.col);
+    v[q][0] = w.x;
+    v[q][1] = w.y;
+  }
+}
+
+// the rows a warp's neighbours read: its first and last rows' cells of either colour, as last updated
+struct MgEdges {
+  float lo[2][kMgWarps + 2][32], hi[2][kMgWarps + 2][32];  // warp w is entry w + 1
+};
+// a_W x_W + a_S x_S + a_N x_N + a_E x_E of cell s of the pair in row q, summed in that order from zero (a
+// coefficient without a neighbour is zero); up, dn: the cells before the first and after the last row
+template <int Q, int S>
+__device__ __forceinline__ float mg_tile_sum(const MgTile &T, float up, float dn) {
+  const float w = Q == 0 ? up : T.x[Q > 0 ? Q - 1 : 0][S];
+  const float e = Q == kMgRows - 1 ? dn : T.x[Q < kMgRows - 1 ? Q + 1 : Q][S];
+  const float side = S == 0 ? __shfl_up_sync(0xffffffffu, T.x[Q][1], 1) : __shfl_down_sync(0xffffffffu, T.x[Q][0], 1);
+  const float so = S == 0 ? side : T.x[Q][0], no = S == 0 ? T.x[Q][1] : side;
+  float s = 0.0f;
+  s += T.a[Q][0][S] * w;
+  s += T.a[Q][1][S] * so;
+  s += T.a[Q][2][S] * no;
+  s += T.a[Q][3][S] * e;
+  return s;
+}
+// f(row index as a constant) for each of a thread's rows
+template <class F>
+__device__ __forceinline__ void mg_rows(F &&f) {
+  f(std::integral_constant<int, 0>{});
+  f(std::integral_constant<int, 1>{});
+  f(std::integral_constant<int, 2>{});
+  f(std::integral_constant<int, 3>{});
+}
+static_assert(kMgRows == 4, "mg_rows");
+// the rows outside the region (its first and last warps' missing neighbours)
+__device__ __forceinline__ void mg_edges_clear(MgEdges &E) {
+  if (threadIdx.x < 64) {
+    const unsigned c = threadIdx.x >> 5, l = threadIdx.x & 31u;
+    E.hi[c][0][l] = 0.0f;
+    E.lo[c][kMgWarps + 1][l] = 0.0f;
+  }
+}
+// One half sweep: the cells of colour COLOR, (row + column) & 1, where the region's first row is PAR (mod 2).
+// FIRST: the iterate is zero on entry, so the cells take b / diag.
+template <int COLOR, int PAR, bool FIRST>
+__device__ __forceinline__ void mg_tile_smooth(MgTile &T, MgEdges &E) {
+  float up = 0.0f, dn = 0.0f;
+  if (!FIRST) {
+    up = E.hi[COLOR ^ 1][T.warp][T.lane];
+    dn = E.lo[COLOR ^ 1][T.warp + 2][T.lane];
+  }
+  float v[kMgRows];
+  auto cell = [&](auto qc) {
+    constexpr int Q = decltype(qc)::value, S = (Q + PAR + COLOR) & 1;
+    float s = T.b[Q][S];
+    if (!FIRST) s -= mg_tile_sum<Q, S>(T, up, dn);
+    v[Q] = s / T.d[Q][S];
+  };
+  mg_rows(cell);
+#pragma unroll
+  for (int q = 0; q < kMgRows; ++q) T.x[q][(q + PAR + COLOR) & 1] = v[q];
+  E.lo[COLOR][T.warp + 1][T.lane] = v[0];
+  E.hi[COLOR][T.warp + 1][T.lane] = v[kMgRows - 1];
+  __syncthreads();
+}
+
+// Pre-smoothing of level F from a zero iterate, the residual and its restriction into C.b; the iterate goes
+// to F.r.  One CTA per tile of kMgDownRows x kMgDownCols cells.
+__global__ void __launch_bounds__(kMgTileThreads, 3) k_mg_down(MgLevel F, MgLevel C, MgFold fold) {
+  __shared__ MgEdges E;
+  __shared__ float rs[kMgRegionRows][kMgRegionCols];
+  const int ti = (int)blockIdx.y * kMgDownRows, tj = (int)blockIdx.x * kMgDownCols;  // the tile's first cell
+  const int i0 = ti - kMgDownRow, j0 = tj - kMgDownCol;
+  constexpr int kPar = kMgDownRow & 1;
+  MgTile T;
+  mg_tile_operator(T, F, i0, j0, fold.px, fold.py);
+  pdl_entry();
+  mg_tile_load(T, F.b, F.ny, T.b);
+#pragma unroll
+  for (int q = 0; q < kMgRows; ++q) T.x[q][0] = T.x[q][1] = 0.0f;
+  mg_edges_clear(E);
+  mg_tile_smooth<0, kPar, true>(T, E);
+  mg_tile_smooth<1, kPar, false>(T, E);
+#pragma unroll
+  for (int k = 1; k < kMgSweeps; ++k) {
+    mg_tile_smooth<0, kPar, false>(T, E);
+    mg_tile_smooth<1, kPar, false>(T, E);
+  }
+  auto residual = [&](auto qc) {
+    constexpr int Q = decltype(qc)::value;
+    float r[2];
+    {
+      constexpr int kC = (Q + kPar) & 1;  // colour of cell 0; the rows above and below hold the other one there
+      const float up = Q == 0 ? E.hi[kC ^ 1][T.warp][T.lane] : 0.0f;
+      const float dn = Q == kMgRows - 1 ? E.lo[kC ^ 1][T.warp + 2][T.lane] : 0.0f;
+      r[0] = T.b[Q][0] - (T.d[Q][0] * T.x[Q][0] + mg_tile_sum<Q, 0>(T, up, dn));
+    }
+    {
+      constexpr int kC = (Q + kPar + 1) & 1;
+      const float up = Q == 0 ? E.hi[kC ^ 1][T.warp][T.lane] : 0.0f;
+      const float dn = Q == kMgRows - 1 ? E.lo[kC ^ 1][T.warp + 2][T.lane] : 0.0f;
+      r[1] = T.b[Q][1] - (T.d[Q][1] * T.x[Q][1] + mg_tile_sum<Q, 1>(T, up, dn));
+    }
+    const int row = (int)T.warp * kMgRows + Q;
+    *(float2 *)&rs[row][2 * T.lane] = make_float2(r[0], r[1]);
+    const int i = i0 + row, j = j0 + 2 * (int)T.lane;  // the tile's own cells are inside the level as they stand
+    if (row >= kMgDownRow && row < kMgDownRow + kMgDownRows && i < F.nx && j >= tj && j < tj + kMgDownCols && j < F.ny)
+      *(float2 *)(F.r + (size_t)i * F.ny + j) = make_float2(T.x[Q][0], T.x[Q][1]);
+  };
+  mg_rows(residual);
+  __syncthreads();
+  // coarse cells: a warp a row, a lane a column
+  const int cj = (int)T.lane, J = tj / 2 + cj;
+  if (cj >= kMgDownCols / 2 || J >= C.ny) return;
+  float wx[4], wy[4];
+  mg_w4(J, C.ny, fold.py, fold.s[2], fold.s[3], wy);
+  for (int ci = (int)T.warp; ci < kMgDownRows / 2; ci += kMgWarps) {
+    const int I = ti / 2 + ci;
+    if (I >= C.nx) break;
+    mg_w4(I, C.nx, fold.px, fold.s[0], fold.s[1], wx);
+    const float *f = &rs[kMgDownRow + 2 * ci - 1][kMgDownCol + 2 * cj - 1];
+    C.b[(size_t)I * C.ny + J] = mg_restrict_sum(wx, wy, [&](int p, int q) { return f[p * kMgRegionCols + q]; });
+  }
+}
+
+// x = F.r + P (C.x), post-smoothing of level F; the iterate goes to F.x.  One CTA per tile of kMgUpRows x kMgUpCols
+// cells.
+__global__ void __launch_bounds__(kMgTileThreads, 3) k_mg_up(MgLevel C, MgLevel F, MgFold fold) {
+  constexpr int kCo = kMgRegionCols / 2 + 2, kCr = kMgRegionRows / 2 + 2;  // the coarse cells of the region and one ring
+  __shared__ MgEdges E;
+  __shared__ float cs[kCr][kCo];
+  const int ti = (int)blockIdx.y * kMgUpRows, tj = (int)blockIdx.x * kMgUpCols;
+  const int i0 = ti - kMgUp, j0 = tj - kMgUp;
+  MgTile T;
+  mg_tile_operator(T, F, i0, j0, fold.px, fold.py);
+  pdl_entry();
+  mg_tile_load(T, F.b, F.ny, T.b);
+  mg_tile_load(T, F.r, F.ny, T.x);
+  for (int t = (int)threadIdx.x; t < kCr * kCo; t += kMgTileThreads) {
+    const int ci = t / kCo, cj = t - ci * kCo;
+    int I = i0 / 2 - 1 + ci, J = j0 / 2 - 1 + cj;
+    // a missing parent at a wall is the boundary cell itself, with weight zero
+    I = fold.px ? mg_wrap(I, C.nx, 1) : min(max(I, 0), C.nx - 1);
+    J = fold.py ? mg_wrap(J, C.ny, 1) : min(max(J, 0), C.ny - 1);
+    cs[ci][cj] = C.x[(size_t)I * C.ny + J];
+  }
+  mg_edges_clear(E);
+  __syncthreads();
+  {
+    float wy[2][2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      wy[s][0] = 0.75f;
+      wy[s][1] = 0.25f;
+      if (!fold.py && T.col + s == (s == 0 ? 0 : F.ny - 1)) {
+        wy[s][0] += 0.25f * (s == 0 ? fold.s[2] : fold.s[3]);
+        wy[s][1] = 0.0f;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kMgRows; ++q) {
+      const bool in = T.row[q] >= 0 && T.col >= 0;
+      const int o = q & 1;  // the region's first row and a warp's rows are even
+      float wx[2] = {0.75f, 0.25f};
+      if (!fold.px && T.row[q] == (o == 0 ? 0 : F.nx - 1)) {
+        wx[0] += 0.25f * (o == 0 ? fold.s[0] : fold.s[1]);
+        wx[1] = 0.0f;
+      }
+      const int I[2] = {((int)T.warp * kMgRows + q) / 2 + 1, ((int)T.warp * kMgRows + q) / 2 + (o ? 2 : 0)};
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int J[2] = {(int)T.lane + 1, (int)T.lane + (s ? 2 : 0)};
+        float v = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) v += wx[a] * wy[s][b] * cs[I[a]][J[b]];
+        T.x[q][s] = in ? T.x[q][s] + v : 0.0f;
+      }
+    }
+  }
+  // the red cells of the edge rows, which the first half sweep (black) reads
+  E.lo[0][T.warp + 1][T.lane] = T.x[0][0];
+  E.hi[0][T.warp + 1][T.lane] = T.x[kMgRows - 1][(kMgRows - 1) & 1];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kMgSweeps; ++k) {
+    mg_tile_smooth<1, 0, false>(T, E);
+    mg_tile_smooth<0, 0, false>(T, E);
+  }
+#pragma unroll
+  for (int q = 0; q < kMgRows; ++q) {
+    const int row = (int)T.warp * kMgRows + q, i = i0 + row, j = j0 + 2 * (int)T.lane;
+    if (row >= kMgUp && row < kMgUp + kMgUpRows && i < F.nx && j >= tj && j < tj + kMgUpCols && j < F.ny)
+      *(float2 *)(F.x + (size_t)i * F.ny + j) = make_float2(T.x[q][0], T.x[q][1]);
+  }
+}
+
+// The bottom of the V-cycle in one CTA: levels first .. last-1 (the first at most kMgSmemCells cells, so at
+// most kMgBottomLevels levels above the coarsest) smoothed, restricted, the coarsest (last) solved with its
+// inverse, then prolonged and smoothed back up to `first`.  One such launch takes the place of two per level,
+// which at these sizes cost their latency and nothing else.  A thread holds the operator rows of one pair of
+// cells per level in registers, the vectors and the coarsest inverse are in shared memory, and every load of
+// operators is issued before the first phase; the phases then cost a barrier and shared-memory latency each.
 struct MgChain {
   MgLevel lv[kMgMaxLevels];
   int first, last;
   MgFold fold;
   const float *inv;
 };
-__global__ void __launch_bounds__(1024) k_mg_bottom(MgChain Ch) {
+constexpr int kMgSmemCells = 2048;  // a pair per thread
+constexpr int kMgBottomLevels = 2;
+constexpr int kMgBottomThreads = kMgSmemCells / 2;
+static_assert(kMgSmemCells <= kMgCoarseMax << (2 * kMgBottomLevels), "smoothed levels of the bottom");
+// dynamic shared memory: the coarsest inverse, then x, b, r of every level
+constexpr size_t kMgBottomSmem = sizeof(float) * ((size_t)kMgCoarseMax * kMgCoarseMax + 3 * 2 * (size_t)kMgSmemCells);
+
+// One pair of cells of a bottom level, by colour: operator rows and where the neighbours' values are
+struct MgPair {
+  float a[2][4], d[2];
+  int c[2][4];  // the W, S, N, E neighbours' cells (a missing one: the cell itself, coefficient zero)
+  int cell[2];
+  int r, i, j;  // the pair's first cell, its row and column; r < 0: no pair
+};
+__device__ __forceinline__ void mg_pair_load(MgPair &P, const MgLevel &L, int px, int py) {
+  const int n = L.nx * L.ny, half = L.ny >> 1, t = (int)threadIdx.x;
+  P.r = -1;
+  if (2 * t >= n) return;
+  P.i = t / half;
+  P.j = 2 * (t - P.i * half);
+  P.r = P.i * L.ny + P.j;
+  constexpr int ks[4] = {0, 1, 3, 4};
+  float2 v[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) v[k] = __ldg((const float2 *)(L.a + (size_t)k * n + P.r));
+#pragma unroll
+  for (int col = 0; col < 2; ++col) {
+    const int s = (P.i + col) & 1;
+    P.cell[col] = P.r + s;
+    P.d[col] = s ? v[2].y : v[2].x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long c = slot_col<5>(P.i, P.j + s, ks[k], L.nx, L.ny, px, py);
+      P.c[col][k] = c >= 0 ? (int)c : P.cell[col];
+      P.a[col][k] = c >= 0 ? (s ? v[ks[k]].y : v[ks[k]].x) : 0.0f;
+    }
+  }
+}
+__device__ __forceinline__ float mg_pair_sum(const MgPair &P, const float *x, int col) {
+  float v = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v += P.a[col][k] * x[P.c[col][k]];
+  return v;
+}
+template <int COLOR>
+__device__ __forceinline__ void mg_pair_smooth(const MgPair &P, const MgLevel &L) {
+  if (P.r >= 0) L.x[P.cell[COLOR]] = (L.b[P.cell[COLOR]] - mg_pair_sum(P, L.x, COLOR)) / P.d[COLOR];
+  __syncthreads();
+}
+// the parents of fine index i on one side: its own and the neighbour toward it, with their weights
+__device__ __forceinline__ void mg_parents(int i, int nc, int per, float s_lo, float s_hi, int (&I)[2], float (&w)[2]) {
+  I[0] = i >> 1;
+  I[1] = (i & 1) ? I[0] + 1 : I[0] - 1;
+  w[0] = 0.75f;
+  w[1] = 0.25f;
+  const bool lo = I[1] < 0, hi = I[1] >= nc;
+  if (lo || hi) {
+    I[1] = per ? (lo ? nc - 1 : 0) : I[0];
+    if (!per) {
+      w[0] += 0.25f * (lo ? s_lo : s_hi);
+      w[1] = 0.0f;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kMgBottomThreads, 1) k_mg_bottom(const __grid_constant__ MgChain Ch) {
+  extern __shared__ float mg_smem[];
+  const int tid = (int)threadIdx.x, px = Ch.fold.px, py = Ch.fold.py, ns = Ch.last - Ch.first;
+  MgLevel S[kMgBottomLevels + 1];  // the levels with their vectors in shared memory
+  MgPair P[kMgBottomLevels];
+  float *inv = mg_smem, *q = mg_smem + kMgCoarseMax * kMgCoarseMax;
+#pragma unroll
+  for (int k = 0; k <= kMgBottomLevels; ++k) {
+    if (k > ns) continue;
+    S[k] = Ch.lv[Ch.first + k];
+    const int n = S[k].nx * S[k].ny;
+    S[k].x = q;
+    S[k].b = q + n;
+    S[k].r = q + 2 * n;
+    q += 3 * n;
+    if (k < kMgBottomLevels && k < ns) mg_pair_load(P[k], S[k], px, py);
+  }
+  const int nc = Ch.lv[Ch.last].nx * Ch.lv[Ch.last].ny;
+#pragma unroll
+  for (int u = 0; u < kMgCoarseMax * kMgCoarseMax / 4 / kMgBottomThreads; ++u) {  // up to 3 floats past nc^2, inside both
+    const int k = 4 * (tid + u * kMgBottomThreads);
+    if (k < nc * nc) *(float4 *)(inv + k) = __ldg((const float4 *)(Ch.inv + k));
+  }
   pdl_entry();
-  const unsigned tid = threadIdx.x, nt = blockDim.x;
-  const int px = Ch.fold.px, py = Ch.fold.py;
-  for (int l = Ch.first; l < Ch.last; ++l) {
-    const MgLevel &F = Ch.lv[l], &C = Ch.lv[l + 1];
-    const unsigned nf = (unsigned)F.nx * (unsigned)F.ny, nh = nf >> 1, nc = (unsigned)C.nx * (unsigned)C.ny;
-    for (int k = 0; k < kMgSweeps; ++k) {
-      for (unsigned t = tid; t < nh; t += nt) mg_smooth_at(F, 0, k == 0, px, py, t);
-      __syncthreads();
-      for (unsigned t = tid; t < nh; t += nt) mg_smooth_at(F, 1, 0, px, py, t);
-      __syncthreads();
-    }
-    for (unsigned t = tid; t < nf; t += nt) mg_residual_at(F, px, py, t);
-    __syncthreads();
-    for (unsigned t = tid; t < nc; t += nt) mg_restrict_at(F, C, Ch.fold, t);
-    __syncthreads();
-  }
   {
-    const MgLevel &L = Ch.lv[Ch.last];
-    const int n = L.nx * L.ny;
-    for (int i = (int)tid; i < n; i += (int)nt) {  // inv is symmetric: thread i reads column i (coalesced)
-      float s = 0.0f;
-      for (int k = 0; k < n; ++k) s += Ch.inv[(size_t)k * n + i] * L.b[k];
-      L.x[i] = s;
+    const MgLevel &G = Ch.lv[Ch.first];
+    const int n = G.nx * G.ny;
+#pragma unroll
+    for (int u = 0; u < kMgSmemCells / kMgBottomThreads; ++u)
+      if (tid + u * kMgBottomThreads < n) S[0].b[tid + u * kMgBottomThreads] = G.b[tid + u * kMgBottomThreads];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kMgBottomLevels; ++k) {
+    if (k >= ns) continue;
+    const MgLevel &F = S[k], &C = S[k + 1];
+    const MgPair &p = P[k];
+    if (p.r >= 0) {  // red from a zero iterate
+      F.x[p.cell[0]] = F.b[p.cell[0]] / p.d[0];
+      F.x[p.cell[1]] = 0.0f;
+    }
+    __syncthreads();
+    mg_pair_smooth<1>(p, F);
+    for (int m = 1; m < kMgSweeps; ++m) {
+      mg_pair_smooth<0>(p, F);
+      mg_pair_smooth<1>(p, F);
+    }
+    if (p.r >= 0) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        F.r[p.cell[c]] = F.b[p.cell[c]] - (p.d[c] * F.x[p.cell[c]] + mg_pair_sum(p, F.x, c));
+    }
+    __syncthreads();
+    if (tid < C.nx * C.ny) {  // a quarter of a level of kMgSmemCells: fewer cells than threads
+      const int I = tid / C.ny, J = tid - I * C.ny;
+      float wx[4], wy[4];
+      mg_w4(I, C.nx, px, Ch.fold.s[0], Ch.fold.s[1], wx);
+      mg_w4(J, C.ny, py, Ch.fold.s[2], Ch.fold.s[3], wy);
+      int row[4], col[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {  // a cell across a wall has weight zero: any cell's value serves
+        const int i = 2 * I + u - 1, j = 2 * J + u - 1;
+        row[u] = (px ? (i < 0 ? i + F.nx : (i >= F.nx ? i - F.nx : i)) : min(max(i, 0), F.nx - 1)) * F.ny;
+        col[u] = py ? (j < 0 ? j + F.ny : (j >= F.ny ? j - F.ny : j)) : min(max(j, 0), F.ny - 1);
+      }
+      C.b[tid] = mg_restrict_sum(wx, wy, [&](int u, int w) { return F.r[row[u] + col[w]]; });
     }
     __syncthreads();
   }
-  for (int l = Ch.last - 1; l >= Ch.first; --l) {
-    const MgLevel &F = Ch.lv[l], &C = Ch.lv[l + 1];
-    const unsigned nf = (unsigned)F.nx * (unsigned)F.ny, nh = nf >> 1;
-    for (unsigned t = tid; t < nf; t += nt) mg_prolong_at(C, F, Ch.fold, t);
+#pragma unroll
+  for (int k = 0; k <= kMgBottomLevels; ++k) {  // the coarsest level: inv is symmetric, thread i reads column i
+    if (k != ns || tid >= nc) continue;
+    float s = 0.0f;
+    const float *col = inv + tid, *b = S[k].b;
+#pragma unroll 16
+    for (int m = 0; m < nc; ++m) s += col[m * nc] * b[m];
+    S[k].x[tid] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = kMgBottomLevels - 1; k >= 0; --k) {
+    if (k >= ns) continue;
+    const MgLevel &F = S[k], &C = S[k + 1];
+    const MgPair &p = P[k];
+    if (p.r >= 0) {
+      int I[2], J[2];
+      float wx[2], wy[2];
+      mg_parents(p.i, C.nx, px, Ch.fold.s[0], Ch.fold.s[1], I, wx);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        mg_parents(p.j + s, C.ny, py, Ch.fold.s[2], Ch.fold.s[3], J, wy);
+        float v = 0.0f;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b) v += wx[a] * wy[b] * C.x[I[a] * C.ny + J[b]];
+        F.x[p.r + s] += v;
+      }
+    }
     __syncthreads();
-    for (int k = 0; k < kMgSweeps; ++k) {
-      for (unsigned t = tid; t < nh; t += nt) mg_smooth_at(F, 1, 0, px, py, t);
-      __syncthreads();
-      for (unsigned t = tid; t < nh; t += nt) mg_smooth_at(F, 0, 0, px, py, t);
-      __syncthreads();
+    for (int m = 0; m < kMgSweeps; ++m) {
+      mg_pair_smooth<1>(p, F);
+      mg_pair_smooth<0>(p, F);
     }
   }
+  float *out = Ch.lv[Ch.first].x;
+  const int n = Ch.lv[Ch.first].nx * Ch.lv[Ch.first].ny;
+#pragma unroll
+  for (int u = 0; u < kMgSmemCells / kMgBottomThreads; ++u)
+    if (tid + u * kMgBottomThreads < n) out[tid + u * kMgBottomThreads] = S[0].x[tid + u * kMgBottomThreads];
 }
 
 // Coarse operator of level l+1 from the FP64 slots of level l (see the file header), in FP64 with an FP32 copy.
@@ -526,7 +910,7 @@ __global__ void k_mgcg_ctrl(double *scal, double *rec, double tol, cudaGraphCond
 // separated by cluster barriers (barrier.cluster with release / acquire, which orders the global memory the
 // phases exchange), dot products reduced through distributed shared memory in rank order, so every CTA holds
 // the same scalars and takes the same stopping decision.  One launch per inner solve; nothing waits on
-// another launch or spins.  The cell arithmetic is the per-phase kernels' (mg_*_at), phase for phase.
+// another launch or spins.  Every cell sees the operations of k_mg_down, k_mg_bottom and k_mg_up, phase for phase.
 // ---------------------------------------------------------------------------------------------------
 constexpr int kMgClusterThreads = 1024;
 constexpr int kMgClusterMax = 8;              // CTAs per cluster at most (the portable cluster size)
@@ -578,9 +962,9 @@ __device__ __forceinline__ void mgc_sum(double (&v)[K], double *sh, double (*slo
   par ^= 1;
 }
 
-// The off-diagonal sum of mg_row_sum for up to kMgBatch cells at once: every load of the batch is issued
+// The off-diagonal sums a_s x_nb of up to kMgBatch cells at once: every load of the batch is issued
 // before any sum is formed (the neighbours' x values do not wait for the coefficients), then each cell's sum
-// is taken in slot order over its non-zero coefficients, as mg_row_sum takes it.
+// is taken in slot order over its non-zero coefficients.
 constexpr int kMgBatch = 4;
 __device__ __forceinline__ void mg_row_sums(const MgLevel &L, const float *x, const int (&ci)[kMgBatch],
                                             const int (&cj)[kMgBatch], const bool (&on)[kMgBatch], long long n,
@@ -598,7 +982,7 @@ __device__ __forceinline__ void mg_row_sums(const MgLevel &L, const float *x, co
         const long long c = slot_col<5>(ci[u], cj[u], ks[q], L.nx, L.ny, px, py);
         av[u][q] = __ldg(&L.a[(size_t)ks[q] * n + r]);
         if (c >= 0) xv[u][q] = x[c];
-        else av[u][q] = 0.0f;  // mg_row_sum skips a missing neighbour
+        else av[u][q] = 0.0f;  // a missing neighbour is skipped
       }
     }
   }
@@ -612,8 +996,10 @@ __device__ __forceinline__ void mg_row_sums(const MgLevel &L, const float *x, co
   }
 }
 
-// mg_smooth_at for the cells t0, t0 + st, ... (kMgBatch of them, those below lim): one colour, so no cell of
-// the batch reads another's x, and all loads go before the stores.  The arithmetic is mg_smooth_at's.
+// Red-black Gauss-Seidel half sweep at the colour's cells t0, t0 + st, ... (kMgBatch of them, those below lim;
+// (i + j) & 1 == color, ny is even on every smoothed level, so each row holds ny / 2 cells of each colour): no
+// cell of the batch reads another's x, and all loads go before the stores.  first: the iterate is zero on entry,
+// so the colour's cells take b / diag and the other colour's cells are set to zero.
 __device__ __forceinline__ void mg_smooth_batch(const MgLevel &L, int color, int first, int px, int py, unsigned t0,
                                                 unsigned st, unsigned lim) {
   const int half = L.ny >> 1;
@@ -644,7 +1030,7 @@ __device__ __forceinline__ void mg_smooth_batch(const MgLevel &L, int color, int
   }
 }
 
-// mg_residual_at for a batch of cells, loads before stores (r is written, x only read)
+// r = b - A x for a batch of cells, loads before stores (r is written, x only read)
 __device__ __forceinline__ void mg_residual_batch(const MgLevel &L, int px, int py, unsigned t0, unsigned st,
                                                   unsigned lim) {
   const long long n = (long long)L.nx * L.ny;
