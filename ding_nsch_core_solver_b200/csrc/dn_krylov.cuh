@@ -674,151 +674,205 @@ __device__ void apply_levels13_ring(const PcgArgs &P, double m_r, double (&acc)[
   }
 }
 
-// 13-point ILDLT/ICC sweeps with periodic y, where the dependency graph is one chain over all rows in
-// natural order.  The chain is only carried along a line: a row's lower neighbours in earlier lines were
-// finished with those lines, and in the reference's ascending column order they come before its same-line
-// neighbours (its upper neighbours in later lines come after them).  So, per line, all threads of CTA 0
-// first gather everything a row needs into shared memory -- its earlier-line sum (forward) or later-line
-// products (backward), and the coefficients and offsets of its same-line neighbours -- and thread 0 then
-// runs the line's recurrence from shared memory alone, interior rows (2 <= j < ny-2, same-line neighbours
-// j-1, j-2 / j+1, j+2) with the previous values in registers.  Every row performs the same operations in the
-// same order as apply_levels, so the results are identical.
-constexpr int kSeqSame = 4;   // same-line neighbours of a row, at most (wrap rows)
-constexpr int kSeqLater = 8;  // later-line upper neighbours of a row, at most (periodic x)
-__host__ __device__ constexpr int seq13_smem_doubles_per_row() { return 5 + 2 * kSeqSame + kSeqLater; }
+// 13-point ILDLT/ICC sweeps with periodic y, where the dependency graph is one chain over all rows in natural
+// order.  The chain is only carried along a line: what a row takes from other lines is known before its line
+// begins.  So, per line, CTA 0's threads form those sums in shared memory, and one warp runs the recurrence of
+// the line, y_j = s_j - l2_j y_{j-2} - l1_j y_{j-1} (backward likewise from the other end), with the previous
+// values in registers and the next rows' operands loaded ahead, while the other warps bring the next line's
+// factor rows into the other half of the buffer.  The rows whose neighbours wrap around (the last two forward,
+// the first two backward) take those terms before the recurrence's.
+//
+// What bounds it: one multiply and one subtract of the chain per row and sweep, about 20 cycles, 0.65 us per
+// line of 64, and about 0.25 us per line for the sums and two barriers.  One thread that gathered a row's
+// neighbours by their number took 127 ns per row and 6.5 us per line; a solve at 64 x 64 cells took 4.51 ms and takes
+// 0.43 ms.
+//
+// nx, ny >= 8 (every handle's), so a row's neighbours are distinct and those across the wrap are apart from those
+// beside it.
+constexpr int kSeqCoef = 9;  // per row and buffer: 4 coefficients of other lines, l2, l1, dinv, the sum, r
+constexpr int kSeqChunk = 4;
+__host__ __device__ constexpr int seq13_smem_doubles_per_row() { return 2 * kSeqCoef + 3; }
 
+// One line's recurrence, rows first, first + dir, ...: v_j = s_j - c2_j v_{j-2 dir} - c1_j v_{j-dir} (times dv_j
+// for ICC).  x: the coefficients of the wrap terms of the last two rows: x[0] of the line's first row in the
+// last but one, x[1] and x[2] of the first and second in the last.
+template <bool ICC, int DIR>
+__device__ __forceinline__ void seq13_chain(const double *s, const double *c2, const double *c1, const double *dv,
+                                            double *v, int ny, const double *x) {
+  const int first = DIR > 0 ? 0 : ny - 1, m = ny - 2;
+  double pm2 = 0.0, pm1 = 0.0, v0 = 0.0, v1 = 0.0;
+  double ns[kSeqChunk], n2[kSeqChunk], n1[kSeqChunk], nd[kSeqChunk];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int k = 0; k < kSeqChunk; ++k) {
+      const int j = first + DIR * min(k0 + k, ny - 1);
+      ns[k] = s[j];
+      n2[k] = c2[j];
+      n1[k] = c1[j];
+      nd[k] = ICC ? dv[j] : 1.0;
+    }
+  };
+  auto row = [&](int k, double a, double b2, double b1, double d) {
+    double t = a - b2 * pm2;
+    t = t - b1 * pm1;
+    if (ICC) t = t * d;
+    v[first + DIR * k] = t;
+    pm2 = pm1;
+    pm1 = t;
+  };
+  load(0);
+  int k0 = 0;
+  for (; k0 + kSeqChunk <= m; k0 += kSeqChunk) {
+    double as[kSeqChunk], a2[kSeqChunk], a1[kSeqChunk], ad[kSeqChunk];
+#pragma unroll
+    for (int k = 0; k < kSeqChunk; ++k) {
+      as[k] = ns[k];
+      a2[k] = n2[k];
+      a1[k] = n1[k];
+      ad[k] = nd[k];
+    }
+    load(k0 + kSeqChunk);
+#pragma unroll
+    for (int k = 0; k < kSeqChunk; ++k) {
+      row(k0 + k, as[k], a2[k], a1[k], ad[k]);
+      if (k0 == 0 && k == 0) v0 = pm1;
+      if (k0 == 0 && k == 1) v1 = pm1;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kSeqChunk - 1; ++k)
+    if (k0 + k < m) row(k0 + k, ns[k], n2[k], n1[k], nd[k]);
+  const int e = first + DIR * m, g = first + DIR * (m + 1);
+  row(m, s[e] - x[0] * v0, c2[e], c1[e], ICC ? dv[e] : 1.0);
+  row(m + 1, (s[g] - x[1] * v0) - x[2] * v1, c2[g], c1[g], ICC ? dv[g] : 1.0);
+}
+
+template <bool ICC>
 __device__ void apply_seq13(const PcgArgs &P, double m_r, double (&acc)[3], double *sm) {
-  constexpr int S = 13;
   const SpOp &A = P.A;
-  const int n = A.n, nx = A.nx, ny = A.ny;
-  const bool icc = P.prec == kPrecICC;
-  double *part = sm;                  // earlier-line sum (forward) / y or y D^-1 (backward)
-  double *dv = sm + ny;               // dinv
-  double *ln = sm + 2 * ny;           // the current line's y (forward) or z (backward)
-  double *ns = sm + 3 * ny;           // number of same-line neighbours (then of later-line products)
-  double *sc = sm + 4 * ny;           // [kSeqSame][ny] same-line coefficients, ascending column
-  int *so = (int *)(sm + (4 + kSeqSame) * ny);  // [kSeqSame][ny] their columns j'
-  double *q = sm + (4 + 2 * kSeqSame) * ny;     // [kSeqLater][ny] backward: later-line products, ascending column
-  double *rr = sm + (4 + 2 * kSeqSame + kSeqLater) * ny;  // backward: r of the line
-  // ---- forward: y_r = (r_r - m - sum_{lower, ascending} L y) (* dinv for ICC)
+  const int nx = A.nx, ny = A.ny, px = A.px, nt = (int)blockDim.x, tid = (int)threadIdx.x;
+  const size_t n = (size_t)A.n;
+  auto buf = [&](int i, int k) { return sm + ((size_t)(i & 1) * kSeqCoef + k) * ny; };
+  auto ring = [&](int i) { return sm + (size_t)(2 * kSeqCoef + (i + 3) % 3) * ny; };
+  __shared__ double wrap[2][3];
+  // ---- forward: y_r = (r_r - m - sum_{lower} L y) (* dinv for ICC)
+  auto load_f = [&](int i, int t0, int st) {
+    if (i >= nx) return;
+    const size_t base = (size_t)i * ny;
+    for (int j = t0; j < ny; j += st) {
+      const size_t r = base + j;
+      double c[7];
+#pragma unroll
+      for (int s = 0; s < 6; ++s) c[s] = P.l[s * n + r];
+      c[6] = P.dinv[r];
+      const double rv = P.r[r] - m_r;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) buf(i, s)[j] = c[s];
+      buf(i, 4)[j] = j >= 2 ? c[4] : 0.0;
+      buf(i, 5)[j] = j >= 1 ? c[5] : 0.0;
+      buf(i, 6)[j] = c[6];
+      buf(i, 7)[j] = rv;
+    }
+    if (t0 == st - 1) {
+      wrap[i & 1][0] = P.l[8 * n + base + ny - 2];
+      wrap[i & 1][1] = P.l[7 * n + base + ny - 1];
+      wrap[i & 1][2] = P.l[8 * n + base + ny - 1];
+    }
+  };
+  load_f(0, tid, nt);
+  __syncthreads();
   for (int i = 0; i < nx; ++i) {
-    const long long base = (long long)i * ny;
-    for (int j = threadIdx.x; j < ny; j += blockDim.x) {
-      const long long r = base + j;
-      int slots[S];
-      long long cols[S];
-      const int cnt = lower_slots<S>(A, i, j, slots, cols);
-      double sum = P.r[r] - m_r;
-      int p = 0;
-      for (; p < cnt && cols[p] < base; ++p) sum -= P.l[(size_t)slots[p] * n + r] * P.y[cols[p]];
-      part[j] = sum;
-      int k = 0;
-      for (; p < cnt && k < kSeqSame; ++p, ++k) {
-        sc[(size_t)k * ny + j] = P.l[(size_t)slots[p] * n + r];
-        so[(size_t)k * ny + j] = (int)(cols[p] - base);
+    const size_t base = (size_t)i * ny;
+    double *sum = buf(i, 7);
+    const double *b1 = ring(i - 1), *b2 = ring(i - 2);
+    for (int j = tid; j < ny; j += nt) {
+      const int jm = j > 0 ? j - 1 : ny - 1, jp = j < ny - 1 ? j + 1 : 0;
+      double s = sum[j];
+      if (px && i == nx - 1)
+        s = ((s - P.l[9 * n + base + j] * P.y[jm]) - P.l[10 * n + base + j] * P.y[j]) - P.l[11 * n + base + j] * P.y[jp];
+      if (px && i >= nx - 2) s -= P.l[12 * n + base + j] * P.y[(size_t)(i + 2 - nx) * ny + j];
+      if (i >= 2) s -= buf(i, 0)[j] * b2[j];
+      if (i >= 1) {
+        s = ((s - buf(i, 1)[j] * b1[jm]) - buf(i, 2)[j] * b1[j]) - buf(i, 3)[j] * b1[jp];
+        P.y[base - ny + j] = b1[j];
       }
-      ns[j] = (double)k;
-      dv[j] = P.dinv[r];
+      sum[j] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      auto general = [&](int j) -> double {
-        double sum = part[j];
-        const int k = (int)ns[j];
-        for (int t = 0; t < k; ++t) sum -= sc[(size_t)t * ny + j] * ln[so[(size_t)t * ny + j]];
-        const double yv = icc ? sum * dv[j] : sum;
-        ln[j] = yv;
-        P.y[base + j] = yv;
-        return yv;
-      };
-      double ym2 = general(0);  // y(i, j-2)
-      double ym1 = general(1);  // y(i, j-1)
-#pragma unroll 4
-      for (int j = 2; j < ny - 2; ++j) {
-        // same-line neighbours (i, j-2), (i, j-1) in that order; an absent one has coefficient 0 here and
-        // is skipped by apply_levels: subtracting 0 * y leaves the sum unchanged
-        const int kk = (int)ns[j];
-        const double l2 = kk == 2 ? sc[j] : ((kk == 1 && so[j] == j - 2) ? sc[j] : 0.0);
-        const double l1 = kk == 2 ? sc[(size_t)ny + j] : ((kk == 1 && so[j] == j - 1) ? sc[j] : 0.0);
-        double sum = part[j];
-        sum -= l2 * ym2;
-        sum -= l1 * ym1;
-        const double yv = icc ? sum * dv[j] : sum;
-        ln[j] = yv;
-        P.y[base + j] = yv;
-        ym2 = ym1;
-        ym1 = yv;
-      }
-      general(ny - 2);
-      general(ny - 1);
-    }
+    if (tid < 32)
+      seq13_chain<ICC, 1>(sum, buf(i, 4), buf(i, 5), buf(i, 6), ring(i), ny, wrap[i & 1]);
+    else
+      load_f(i + 1, tid - 32, nt - 32);
     __syncthreads();
   }
-  // ---- backward: z_r = y_r (/D) - sum_{c > r ascending} L_cr z_c (* dinv for ICC); rows in descending order
+  for (int j = tid; j < ny; j += nt) P.y[(size_t)(nx - 1) * ny + j] = ring(nx - 1)[j];
+  __syncthreads();
+  // ---- backward: z_r = y_r (/D) - sum_{c > r} L_cr z_c (* dinv for ICC); lines and rows in descending order
+  auto load_b = [&](int i, int t0, int st) {
+    if (i < 0) return;
+    const size_t base = (size_t)i * ny;
+    for (int j = t0; j < ny; j += st) {
+      const size_t r = base + j;
+      const int jm = j > 0 ? j - 1 : ny - 1, jp = j < ny - 1 ? j + 1 : 0;
+      double c[6];
+      c[0] = i + 2 < nx ? P.l[r + 2 * (size_t)ny] : 0.0;
+      c[1] = i + 1 < nx ? P.l[3 * n + base + ny + jm] : 0.0;
+      c[2] = i + 1 < nx ? P.l[2 * n + base + ny + j] : 0.0;
+      c[3] = i + 1 < nx ? P.l[n + base + ny + jp] : 0.0;
+      c[4] = j + 2 < ny ? P.l[4 * n + r + 2] : 0.0;
+      c[5] = j + 1 < ny ? P.l[5 * n + r + 1] : 0.0;
+      const double d = P.dinv[r], y = P.y[r], rv = P.r[r];
+#pragma unroll
+      for (int s = 0; s < 6; ++s) buf(i, s)[j] = c[s];
+      buf(i, 6)[j] = d;
+      buf(i, 7)[j] = ICC ? y : y * d;
+      buf(i, 8)[j] = rv;
+    }
+    if (t0 == st - 1) {
+      wrap[i & 1][0] = P.l[8 * n + base + ny - 1];
+      wrap[i & 1][1] = P.l[7 * n + base + ny - 1];
+      wrap[i & 1][2] = P.l[8 * n + base + ny - 2];
+    }
+  };
+  auto leave = [&](int i, int j) {  // z of a finished line, and its part of the sums
+    const double zv = ring(i)[j], rv = buf(i, 8)[j] - m_r;
+    P.z[(size_t)i * ny + j] = zv;
+    acc[0] += zv;
+    acc[1] += rv * zv;
+    acc[2] += rv;
+  };
+  load_b(nx - 1, tid, nt);
+  __syncthreads();
   for (int i = nx - 1; i >= 0; --i) {
-    const long long base = (long long)i * ny;
-    for (int j = threadIdx.x; j < ny; j += blockDim.x) {
-      const long long r = base + j;
-      int slots[S];
-      long long cols[S];
-      int cnt = 0;
-      for (int s = 0; s < S; ++s) {
-        const long long c = slot_col<S>(i, j, s, A.nx, A.ny, A.px, A.py);
-        if (c <= r) continue;
-        if (P.l[(size_t)(S - 1 - s) * n + c] == 0.0) continue;
-        int p = cnt++;
-        while (p > 0 && cols[p - 1] > c) {
-          cols[p] = cols[p - 1];
-          slots[p] = slots[p - 1];
-          --p;
-        }
-        cols[p] = c;
-        slots[p] = s;
+    const size_t last = (size_t)(nx - 1) * ny;
+    double *sum = buf(i, 7);
+    const double *b1 = ring(i + 1), *b2 = ring(i + 2);
+    for (int j = tid; j < ny; j += nt) {
+      const int jm = j > 0 ? j - 1 : ny - 1, jp = j < ny - 1 ? j + 1 : 0;
+      double s = sum[j];
+      if (px && i == 0)
+        s = ((s - P.l[11 * n + last + jm] * P.z[last + jm]) - P.l[10 * n + last + j] * P.z[last + j]) -
+            P.l[9 * n + last + jp] * P.z[last + jp];
+      if (px && i < 2) {
+        const size_t c = (size_t)(i - 2 + nx) * ny + j;
+        s -= P.l[12 * n + c] * P.z[c];
       }
-      int p = 0, k = 0;
-      for (; p < cnt && cols[p] < base + ny && k < kSeqSame; ++p, ++k) {
-        sc[(size_t)k * ny + j] = P.l[(size_t)(S - 1 - slots[p]) * n + cols[p]];
-        so[(size_t)k * ny + j] = (int)(cols[p] - base);
-      }
-      int t = 0;
-      for (; p < cnt && t < kSeqLater; ++p, ++t)
-        q[(size_t)t * ny + j] = P.l[(size_t)(S - 1 - slots[p]) * n + cols[p]] * P.z[cols[p]];
-      ns[j] = (double)(k + 16 * t);  // same-line count + 16 x later-line count
-      part[j] = icc ? P.y[r] : P.y[r] * P.dinv[r];
-      dv[j] = P.dinv[r];
-      rr[j] = P.r[r];
+      if (i + 2 < nx) s -= buf(i, 0)[j] * b2[j];
+      if (i + 1 < nx) s = ((s - buf(i, 1)[j] * b1[jm]) - buf(i, 2)[j] * b1[j]) - buf(i, 3)[j] * b1[jp];
+      sum[j] = s;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double zp1 = 0.0, zp2 = 0.0;  // z(i, j+1), z(i, j+2)
-      for (int j = ny - 1; j >= 0; --j) {
-        const int code = (int)ns[j];
-        const int k = code & 15, t = code >> 4;
-        double sum = part[j];
-        if (j >= 2 && j < ny - 2) {
-          // same-line neighbours (i, j+1), (i, j+2) in that order (coefficient 0 when absent)
-          const double e1 = (k >= 1 && so[j] == j + 1) ? sc[j] : 0.0;
-          const double e2 = (k == 2) ? sc[(size_t)ny + j] : ((k == 1 && so[j] == j + 2) ? sc[j] : 0.0);
-          sum -= e1 * zp1;
-          sum -= e2 * zp2;
-        } else {
-          for (int u = 0; u < k; ++u) sum -= sc[(size_t)u * ny + j] * ln[so[(size_t)u * ny + j]];
-        }
-        for (int u = 0; u < t; ++u) sum -= q[(size_t)u * ny + j];
-        const double zv = icc ? sum * dv[j] : sum;
-        ln[j] = zv;
-        const long long r = base + j;
-        P.z[r] = zv;
-        const double rv = rr[j] - m_r;
-        acc[0] += zv;
-        acc[1] += rv * zv;
-        acc[2] += rv;
-        zp2 = zp1;
-        zp1 = zv;
-      }
+    if (tid < 32) {
+      seq13_chain<ICC, -1>(sum, buf(i, 4), buf(i, 5), buf(i, 6), ring(i), ny, wrap[i & 1]);
+    } else {
+      if (i + 1 < nx)
+        for (int j = tid - 32; j < ny; j += nt - 32) leave(i + 1, j);
+      load_b(i - 1, tid - 32, nt - 32);
     }
     __syncthreads();
   }
+  for (int j = tid; j < ny; j += nt) leave(0, j);
+  __syncthreads();
 }
 
 // One persistent launch runs the whole PCG.  SWEEP: 0 = 5-point pipelined wavefront on global memory,
@@ -1019,8 +1073,10 @@ __global__ void __launch_bounds__(kBlock) k_pcg(PcgArgsT<T> P) {
         if (blockIdx.x == 0) {
           if (S == 13 && P.rows13.lval != nullptr && P.rows13.k == 6)
             apply_levels13_ring<6>(P, m_r_now, acc, (double *)dsm);
+          else if (S == 13 && P.seq_lines && P.prec == kPrecICC)
+            apply_seq13<true>(P, m_r_now, acc, (double *)dsm);
           else if (S == 13 && P.seq_lines)
-            apply_seq13(P, m_r_now, acc, (double *)dsm);
+            apply_seq13<false>(P, m_r_now, acc, (double *)dsm);
           else
             apply_levels<S>(P, m_r_now, acc);
         }
