@@ -135,8 +135,9 @@ __global__ void k_outer_residual(SpOp A, const double *b, const double *x, doubl
   pdl_entry();
   __shared__ double sh[3 * 32];
   double v[3] = {0.0, 0.0, 0.0};
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < A.n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / A.ny), j = (int)(t % A.ny);
+  const unsigned n = (unsigned)A.n, ny = (unsigned)A.ny;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const int i = (int)(t / ny), j = (int)(t - (unsigned)i * ny);
     const double rr = b[t] - spmv_row<S>(A, x, i, j);
     r[t] = rr;
     v[0] += rr;
@@ -1553,6 +1554,12 @@ dn_status capture_exec(dn_handle *h, cudaGraphExec_t *exec, Record &&record) {
   return DN_OK;
 }
 
+// CTAs of the mixed form's FP64 residual and correction passes (each leaves three partial sums).  With 128 of
+// them a 1024 x 2048 grid was 64 rows a thread one after another: 590 us for the 13-point residual.
+int mixed_sum_blocks(const dn_handle *h) {
+  return (int)std::min<long long>({(long long)kMaxBlocks, 4LL * h->num_sms, (long long)blocks_for(h->n)});
+}
+
 // One FP32 inner solve A e = b by CG preconditioned with `vcycles` V-cycles of H applied in sequence (1 for
 // the pressure operator; 2 for the CH operator, preconditioned by (K + s I)^-2), recorded into the capture:
 // r = b, then a while node whose body is one iteration (precondition, r.z, direction, A p, p.q, update,
@@ -1694,7 +1701,7 @@ dn_status rec_mixed_pressure(dn_handle *h, bool split, int kind, DcNodes *nodes)
   P.ch = 0;
   P.mg_flag = h->mgp.levels() > 0 ? h->mgp.flag : nullptr;
   const SpOp A{h->a5, (int)n, h->G.nx, h->G.ny, h->G.px, h->G.py};
-  const int nb = 128;
+  const int nb = mixed_sum_blocks(h);
   DN_CUDA(h, cudaMemsetAsync(R, 0, kDcSize * sizeof(double), h->stream));
   cudaGraphConditionalHandle loop = 0;
   DN_TRY(cond_create(h, &loop));
@@ -1856,7 +1863,7 @@ dn_status rec_mixed_ch(dn_handle *h, DcNodes *nodes) {
   P.ch = 1;
   P.mg_flag = h->mgc.flag;
   const SpOp A{h->a13, (int)n, h->G.nx, h->G.ny, h->G.px, h->G.py};
-  const int nb = 128;
+  const int nb = mixed_sum_blocks(h);
   DN_CUDA(h, cudaMemsetAsync(R, 0, kDcSize * sizeof(double), h->stream));
   cudaGraphConditionalHandle loop = 0;
   DN_TRY(cond_create(h, &loop));

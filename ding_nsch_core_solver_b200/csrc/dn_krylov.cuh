@@ -65,17 +65,41 @@ struct SpOpT {
 };
 using SpOp = SpOpT<double>;
 
+// (A x)(i, j), the products added in slot order over the non-zero slots.  Every load is issued whatever the
+// coefficients are (a missing neighbour reads the row's own x and is not added): with a branch per slot each
+// x waited for its coefficient, 13 memory latencies one after another per row.
 template <int S, typename T>
 __device__ __forceinline__ T spmv_row(const SpOpT<T> &A, const T *x, int i, int j) {
-  const long long r = (long long)i * A.ny + j;
+  constexpr int R = S == 5 ? 1 : 2;
+  const int r = i * A.ny + j;
+  int row[2 * R + 1], col[2 * R + 1];
+  bool rin[2 * R + 1], cin[2 * R + 1];
+#pragma unroll
+  for (int d = -R; d <= R; ++d) {
+    int ii = i + d, jj = j + d;
+    rin[d + R] = A.px || (ii >= 0 && ii < A.nx);
+    cin[d + R] = A.py || (jj >= 0 && jj < A.ny);
+#pragma unroll
+    for (int w = 0; w < R; ++w) {  // an extent of one wraps twice
+      ii = ii < 0 ? ii + A.nx : (ii >= A.nx ? ii - A.nx : ii);
+      jj = jj < 0 ? jj + A.ny : (jj >= A.ny ? jj - A.ny : jj);
+    }
+    row[d + R] = rin[d + R] ? ii * A.ny : i * A.ny;
+    col[d + R] = cin[d + R] ? jj : j;
+  }
+  T a[S], v[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int u = Stencil<S>::di(s) + R, w = Stencil<S>::dj(s) + R;
+    a[s] = A.a[(size_t)s * A.n + r];
+    v[s] = x[row[u] + col[w]];
+    if (!(rin[u] && cin[w])) a[s] = T(0);
+  }
   T sum = T(0);
 #pragma unroll
   for (int s = 0; s < S; ++s) {
-    const T a = A.a[(size_t)s * A.n + r];
-    if (a != T(0)) {
-      const long long c = slot_col<S>(i, j, s, A.nx, A.ny, A.px, A.py);
-      sum += a * x[c];
-    }
+    const T t = sum + a[s] * v[s];
+    sum = a[s] != T(0) ? t : sum;
   }
   return sum;
 }
