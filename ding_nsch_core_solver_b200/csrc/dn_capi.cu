@@ -762,6 +762,21 @@ dn_status launch_pdl(dn_handle *h, const char *name, void (*kernel)(KArgs...), d
   return check_launch(h, name);
 }
 
+// the incomplete factor of a 5-point operator (F.l zeroed and written): k_factor5 up to its line limit, k_factor
+// beyond; *name: the kernel launched
+void launch_factor5(const SpOp &A, const Factor &F, int kind, int *status, cudaStream_t st, const char **name) {
+  if (A.nx <= kFactorLines) {
+    *name = "k_factor5";
+    cudaMemsetAsync(F.l, 0, 5 * (size_t)A.n * sizeof(double), st);
+    const size_t smem = 2 * (size_t)A.nx * sizeof(double);
+    cudaFuncSetAttribute(k_factor5, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kFactorLines * sizeof(double)));
+    k_factor5<<<1, kFactorThreads, smem, st>>>(A, F, kind, status);
+  } else {
+    *name = "k_factor<5>";
+    k_factor<5><<<1, 1024, 0, st>>>(A, F, kind, status);
+  }
+}
+
 bool is_uish(int id) { return id == DN_F_U || id == DN_F_U_PREV || id == DN_F_U_STAR || id == DN_F_SFX_U || id == DN_F_HU_PREV; }
 bool is_vish(int id) { return id == DN_F_V || id == DN_F_V_PREV || id == DN_F_V_STAR || id == DN_F_SFY_V || id == DN_F_HV_PREV; }
 
@@ -1654,9 +1669,9 @@ dn_status rec_ic32_factor(dn_handle *h, bool split, int kind, double *R, cudaGra
   if (!(split && h->p_factor_valid && h->p_factor_kind == kind)) {
     DN_CUDA(h, cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
     Factor F{h->l5, h->d5, h->dinv5, 0.0};
-    k_factor<5><<<1, 1024, 0, h->stream>>>(SpOp{h->a5, (int)n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F, kind,
-                                            h->status);
-    DN_TRY(check_launch(h, "k_factor<5>"));
+    const char *name = nullptr;
+    launch_factor5(SpOp{h->a5, (int)n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F, kind, h->status, h->stream, &name);
+    DN_TRY(check_launch(h, name));
   } else {
     DN_CUDA(h, cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
   }
@@ -2977,9 +2992,9 @@ dn_status pressure_factor(dn_handle *h, bool split, bool icc) {
   if (!(split && h->p_factor_valid && h->p_factor_kind == kind)) {
     DN_CUDA(h, cudaMemsetAsync(h->status, 0, sizeof(int), h->stream));
     Factor F{h->l5, h->d5, h->dinv5, 0.0};
-    k_factor<5><<<1, 1024, 0, h->stream>>>(SpOp{h->a5, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F, kind,
-                                            h->status);
-    DN_TRY(check_launch(h, "k_factor<5>"));
+    const char *name = nullptr;
+    launch_factor5(SpOp{h->a5, (int)h->n, h->G.nx, h->G.ny, h->G.px, h->G.py}, F, kind, h->status, h->stream, &name);
+    DN_TRY(check_launch(h, name));
     if (h->capturing) {  // recorded: the status goes to the step record (a failed factor is reported after)
       k_rec_copy<<<1, 32, 0, h->stream>>>(nullptr, 0, h->status, h->rec + kRecStep + kSPFactor);
       return check_launch(h, "k_rec_copy");
@@ -5072,8 +5087,9 @@ dn_status dn_pressure_solve_static(const dn_config *cfg, int step, const double 
     DN_SLAUNCH("k_vec_sub_scalar");
   }
   const SpOp A{a5, (int)n, nx, ny, G.px, G.py};
-  k_factor<5><<<1, 1024, 0, st>>>(A, Factor{dptr(L.l5), dptr(L.d5), dptr(L.dinv5), 0.0}, kind, status);
-  DN_SLAUNCH("k_factor<5>");
+  const char *name = nullptr;
+  launch_factor5(A, Factor{dptr(L.l5), dptr(L.d5), dptr(L.dinv5), 0.0}, kind, status, st, &name);
+  DN_SLAUNCH(name);
   int dev_st = 0;
   {
     const dn_status s = static_read(&dev_st, status, sizeof(int), st, err, err_len);

@@ -260,6 +260,106 @@ __global__ void k_factor(SpOp A, Factor F, int kind, int *status) {
   }
 }
 
+// The 5-point factor.  A row's lower neighbours are never neighbours of one another (nx, ny >= 8), so its entries
+// are L_rc = a_rc / max(d_c, floor) and d_r = a_rr - sum L_rc^2 (* d_c for ILDLT) in ascending column order: k_factor's
+// operations without its searches.  One CTA walks the levels i + j as there; a thread keeps a line, so d of the row
+// below is its own previous value, d of the line before comes from shared memory, and a thread's operator rows (and
+// the d across a periodic side, finished at least seven levels earlier) are loaded kFactorAhead levels ahead.
+// What bounds it: per level, a divide, a square root, a divide and a barrier one after another, and 7 scattered
+// accesses per row.  k_factor<5> spent most of a level in loads that waited for one another: the
+// pressure phase of a 96 x 192 step with it took 13.07 ms and takes 12.38 ms, 64 x 64 3.84 and 3.50 ms.
+// A.l is zero on entry.  kind, status: as k_factor.
+constexpr int kFactorThreads = 512;
+constexpr int kFactorAhead = 3;      // levels; the walk looks up to 2 kFactorAhead - 1 ahead, less than nx - 1 and ny - 1
+constexpr int kFactorLines = 4096;   // of k_factor5 at most: two levels of d in shared memory
+struct FactorRow {
+  double w, s, c, n, e, dn, de;
+};
+__global__ void __launch_bounds__(kFactorThreads) k_factor5(SpOp A, Factor F, int kind, int *status) {
+  extern __shared__ double dl[];  // [2][nx]: d of the last two levels, by line
+  __shared__ double shmax[32];
+  const int nx = A.nx, ny = A.ny, tid = (int)threadIdx.x, nt = (int)blockDim.x;
+  const size_t n = (size_t)A.n;
+  double m = 0.0;  // max |diag| (ch_sparse_krylov.hpp:258-263 / 343-348)
+#pragma unroll 8
+  for (int r = tid; r < A.n; r += nt) m = fmax(m, fabs(A.a[2 * n + r]));
+  m = warp_max(m);
+  if ((tid & 31) == 0) shmax[tid >> 5] = m;
+  __syncthreads();
+  m = 0.0;
+  for (int w = 0; w < nt >> 5; ++w) m = fmax(m, shmax[w]);
+  const bool icc = kind == 2;
+  const double floor = icc ? sqrt(fmax(1.0, m) * 1.0e-12) : fmax(1.0, m) * 1.0e-12;
+  const double floor_sq = floor * floor;
+  auto load = [&](int i, int lev, FactorRow &q) {
+    const int j = lev - i;
+    q = FactorRow{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (i >= nx || j < 0 || j >= ny) return;
+    const size_t r = (size_t)i * ny + j;
+    q.c = A.a[2 * n + r];
+    if (i > 0) q.w = A.a[r];
+    if (j > 0) q.s = A.a[n + r];
+    if (A.px && i == nx - 1) {
+      q.e = A.a[4 * n + r];
+      q.de = F.d[j];
+    }
+    if (A.py && j == ny - 1) {
+      q.n = A.a[3 * n + r];
+      q.dn = F.d[r - j];
+    }
+  };
+  auto row = [&](int i, int lev, const FactorRow &q) {
+    const int j = lev - i;
+    if (i >= nx || j < 0 || j >= ny) return;
+    const size_t r = (size_t)i * ny + j;
+    const double *old = dl + ((lev + 1) & 1) * nx;
+    double d = q.c;
+    auto entry = [&](double a, double dc, size_t slot) {  // an entry this small is not one (lower_slots)
+      if (fabs(a) < 1.0e-18) return;
+      const double l = a / max_ref(dc, floor);
+      F.l[slot * n + r] = l;
+      d -= icc ? l * l : l * l * dc;
+    };
+    if (A.px && i == nx - 1) entry(q.e, q.de, 4);
+    if (i > 0) entry(q.w, old[i - 1], 0);
+    if (A.py && j == ny - 1) entry(q.n, q.dn, 3);
+    if (j > 0) entry(q.s, old[i], 1);
+    if (icc) {
+      if (!isfinite(d) || d <= floor_sq) {
+        atomicExch(status, kDevFactorFailed);
+        d = floor_sq * 4.0;
+      }
+      d = sqrt(d);
+    } else if (!isfinite(d) || d <= floor) {
+      atomicExch(status, kDevFactorFailed);
+      d = floor * 2.0;
+    }
+    F.d[r] = d;
+    F.dinv[r] = 1.0 / max_ref(d, floor);
+    dl[(lev & 1) * nx + i] = d;
+  };
+  FactorRow cur[kFactorAhead], nxt[kFactorAhead];
+#pragma unroll
+  for (int g = 0; g < kFactorAhead; ++g) load(tid, g, nxt[g]);
+  for (int lev0 = 0; lev0 < nx + ny - 1; lev0 += kFactorAhead) {
+#pragma unroll
+    for (int g = 0; g < kFactorAhead; ++g) {
+      cur[g] = nxt[g];
+      load(tid, lev0 + kFactorAhead + g, nxt[g]);
+    }
+#pragma unroll
+    for (int g = 0; g < kFactorAhead; ++g) {
+      row(tid, lev0 + g, cur[g]);
+      for (int i = tid + nt; i < nx; i += nt) {  // lines beyond the threads
+        FactorRow q;
+        load(i, lev0 + g, q);
+        row(i, lev0 + g, q);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // Diagonal preconditioner (build_diagonal_preconditioner, ch_sparse_krylov.hpp:421-432).
 template <int S>
 __global__ void k_diag_inverse(SpOp A, double *dinv) {
