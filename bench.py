@@ -80,7 +80,7 @@ def initial_state(cfg: dict, seed: int = 2) -> dict:
     return state
 
 
-PCG_PROFILE = os.path.join(ROOT, "profiles", "k_pcg_5_3_pressure_192x384.txt")
+PCG_PROFILE = os.path.join(ROOT, "profiles", "k_wpcg_pressure_192x384.txt")
 
 
 def pcg_traffic_per_launch():
@@ -486,15 +486,16 @@ def run_ours(args):
                 "frac": round(achieved / peak, 5),
                 "traffic": None if per_it is None else round(per_it * statistics.mean(pcg_its)),
                 "peak_source": peak_kind,
-                "kernel": "k_pcg<5,3> (pressure ICC-PCG, persistent, staged wavefront, one launch per solve)",
+                "kernel": "k_wpcg (pressure ICC-PCG, persistent, vectors in sweep order, one launch per solve)",
                 "algorithmic_bytes_per_launch": bytes_per_launch,
                 "kernel_ms_mean": statistics.mean(pcg_ms)}
-    # The sweeps are a dependency chain of nx + ny - 1 steps each way per iteration: time per dependent step
-    # against the shuffle + FMA chain latency (61 cycles, about 31 ns at 1965 MHz, measured on B200).
-    dep_steps = 2 * (cfg["nx"] + cfg["ny"] - 1) * statistics.mean(pcg_its)
+    # The sweeps are a dependency chain of nx + ny / 2 steps of a pair of columns each way per iteration: time per
+    # dependent step against the latency of a shuffle and two FP64 operations (48 cycles, about 25 ns at 1965 MHz,
+    # measured on B200).
+    dep_steps = 2 * (cfg["nx"] + (cfg["ny"] + 1) // 2) * statistics.mean(pcg_its)
     sweep_ms = statistics.mean(p[10] for p in phases)
     critical_path = {"dependent_sweep_steps_per_launch": round(dep_steps), "sweep_ms_per_launch": round(sweep_ms, 3),
-                     "ns_per_dependent_step": round(sweep_ms * 1e6 / dep_steps, 1), "chain_floor_ns": 31.0}
+                     "ns_per_dependent_step": round(sweep_ms * 1e6 / dep_steps, 1), "chain_floor_ns": 25.0}
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:
@@ -520,7 +521,7 @@ def run_ours(args):
                                    "interface modes 2-8", "grid": [cfg["nx"], cfg["ny"]], "pressure_scheme": "split_icpcg",
                        "pressure_tolerance": 1e-10, "ch_tolerance": 1e-10, "precision": "fp64",
                        "l2": "flushed (512 MB write) between timed steps", "parallelism": f"replicas x{world}",
-                       "launch_shape": launch_shape or "default (512 rows per CTA, sweep warps by shared memory)"},
+                       "launch_shape": launch_shape or "default (512 rows per CTA, one sweep block per CTA)"},
             "iterations_mean": mean_rep,
             "phase_ms_mean": {k: round(statistics.mean(p[i] for p in phases), 4) for i, k in enumerate(
                 ("ch", "momentum", "pressure", "correction", "pressure_pcg_kernel", "ch_pcg_kernel",

@@ -87,7 +87,9 @@ typedef struct {
   int dcdm_history_size, dcdm_max_stored_directions, dcdm_restart_interval; /* config.hpp:72-74 */
   int pcg_rows_per_cta;            /* launch shape of the pressure PCG: rows per CTA of its SpMV / update
                                       phases (0: 512) -- see dn_autotune_pressure */
-  int sweep_warps_per_cta;         /* sweep warps per CTA of the staged wavefront (0: as many as fit, up to 4) */
+  int sweep_warps_per_cta;         /* blocks of 32 lines swept per CTA of the pressure PCG (0: 1; at most 2); the
+                                      wavefront of the grids that it does not take: sweep warps per CTA (0: as
+                                      many as fit, up to 4) */
   int device_wait_limit;           /* polls after which a device-side wait (grid barrier, wavefront hand-over)
                                       gives up and the call returns DN_ERR_TIMEOUT (0: the default, 2^22, well
                                       under a few seconds) */
@@ -333,7 +335,7 @@ dn_status dn_pressure_analysis(dn_handle *h, int step, const char *source_mode);
 /* ---- launch-shape autotuning ----------------------------------------------------------------------------- */
 /* No counterpart in the reference.  Times one pressure solve of the handle's current state (u*, v*, rho_mid,
  * p, p_prev as a step leaves them) for each launch shape -- rows per CTA of the PCG's SpMV / update phases
- * in {256 .. 4096} x sweep warps per CTA of the staged wavefront -- twice, and keeps the fastest of the
+ * in {256 .. 4096} x sweep warps per CTA (sweep_warps_per_cta) -- twice, and keeps the fastest of the
  * second pass on the handle.  Outputs (each may be NULL): the chosen shape and its pressure-solve time. */
 dn_status dn_autotune_pressure(dn_handle *h, int *rows_per_cta, int *sweep_warps_per_cta, double *best_ms);
 
@@ -391,7 +393,7 @@ void *dn_stream(dn_handle *h);
 dn_status dn_last_phase_times(dn_handle *h, double *out);
 /* Device-clock profiling counters of the last pressure solve's wavefront (ns), 4 per sweep warp k:
  * [4k] forward sweep, [4k+1] waits for the neighbouring warp, [4k+2] waits for staged inputs,
- * [4k+3] backward sweep.  `count` <= 64. */
+ * [4k+3] backward sweep; the sweep-order kernel writes [4k] and [4k+3] of its blocks.  `count` <= 64. */
 dn_status dn_profile_counters(dn_handle *h, double *out, int count);
 /* Number of this library's kernels launched since the handle was created. */
 long long dn_kernel_launches(const dn_handle *h);
