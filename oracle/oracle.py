@@ -189,7 +189,7 @@ def build(force: bool = False) -> None:
     """Compile the checkers with oracle/Makefile (the reference harness only where the reference exists)."""
     targets = ["oracle"]
     ref = os.environ.get("DN_REFERENCE", "")
-    if ref and os.path.isdir(ref):
+    if ref and os.path.isdir(os.path.join(ref, "src")):
         targets.append("ref")
         if os.path.exists(os.path.join(os.path.dirname(HERE), "ding_nsch_core_solver_b200", "libdn_cuda.so")):
             targets.append("refcuda")
