@@ -357,7 +357,8 @@ __device__ __forceinline__ bool c_help(const CArgs &C, const CWarp &W, long long
       if (has_in && q >= 0 && q < np) st_pair_if(e1 + q, none, true);
       if (wraps && qx - 1 >= 0 && qx - 1 < np) st_pair_if(x0 + qx - 1, none, true);
       if (wraps && qx >= 0 && qx < np) st_pair_if(x1 + qx, none, true);
-      if (wraps && qx == np - 1) st_pair_if(x0 + qx, none, true);
+      // the last entry is looked at once more by the step after (which may come in a later round), if there is one
+      if (wraps && qx == np - 1 && n == S - 1) st_pair_if(x0 + qx, none, true);
     }
     if (count > 0) {
       told = min(told + count, S);
