@@ -120,10 +120,11 @@ __device__ __forceinline__ void block_sum(double (&v)[K], double *sh) {
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += sh[k * 32 + w];
-    v[k] = s;
+  for (int k = 0; k < K; ++k) v[k] = 0.0;
+#pragma unroll 4
+  for (int w = 0; w < nw; ++w) {  // all K at once: one value after another waits K times for as many loads
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] += sh[k * 32 + w];
   }
   __syncthreads();
 }
@@ -185,12 +186,18 @@ __device__ __forceinline__ bool grid_sum(double (&v)[K], double *partials_base, 
   // warp 0 re-adds the partials in a fixed order (lane-strided, then a fixed butterfly; lane 0's value is
   // used), so every CTA obtains the same bits.
   if (threadIdx.x < 32) {
+    double s[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k] = 0.0;
+#pragma unroll 4
+    for (unsigned int b = threadIdx.x; b < bar.nblocks; b += 32) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) s[k] += __ldcg(&partials[(size_t)b * K + k]);
+    }
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-      double s = 0.0;
-      for (unsigned int b = threadIdx.x; b < bar.nblocks; b += 32) s += __ldcg(&partials[(size_t)b * K + k]);
-      s = warp_sum(s);
-      if (threadIdx.x == 0) sh[k] = s;
+      s[k] = warp_sum(s[k]);
+      if (threadIdx.x == 0) sh[k] = s[k];
     }
   }
   __syncthreads();

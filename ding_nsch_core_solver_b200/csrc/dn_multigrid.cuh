@@ -38,7 +38,7 @@ constexpr int kMgCoarseMax = 128;  // cells of the directly inverted coarsest le
 constexpr int kMgMaxLevels = 24;
 constexpr int kMgParts = 1024;     // CTAs of the CG vector kernels at most (per-CTA partial sums)
 constexpr int kMgSweeps = 2;       // red-black sweeps before and after each coarse correction
-constexpr int kMgBottomCells = 8192;  // levels this small run inside the one-CTA bottom kernel
+constexpr int kMgBottomCells = 8192;  // levels this small run on one CTA of the cluster form (k_mgcg_cluster)
 
 // one level of the hierarchy: operator slots [5][n] (W,S,C,N,E), iterate, right-hand side, residual
 struct MgLevel {
@@ -903,9 +903,8 @@ __global__ void k_mgcg_ctrl(double *scal, double *rec, double tol, cudaGraphCond
 }
 
 // ---------------------------------------------------------------------------------------------------
-// The inner CG as one thread-block cluster (level-0 grids up to mg_cluster_cells cells).  Small grids leave a
-// full-device launch per phase latency-bound: a V-cycle is about 11 launches per level, each a few
-// microseconds for a few thousand cells.  Here 1-8 CTAs of 1024 threads, which the hardware schedules
+// The inner CG as one thread-block cluster (level-0 grids up to mg_cluster_cells cells).  Small grids leave
+// every launch of a V-cycle latency-bound, a few microseconds for a few thousand cells.  Here 1-8 CTAs of 1024 threads, which the hardware schedules
 // together, run every iteration of the solve: V-cycles, r.z, direction, A p, p.q and the update as phases
 // separated by cluster barriers (barrier.cluster with release / acquire, which orders the global memory the
 // phases exchange), dot products reduced through distributed shared memory in rank order, so every CTA holds
