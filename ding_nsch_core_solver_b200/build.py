@@ -15,7 +15,9 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libdn_cuda.so")
 SOURCES = ["dn_capi.cu", "dn_config.cpp"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-split-compile=0", "-lineinfo", "--fmad=false", "-std=c++17",
+# No -split-compile: with it the kernels' code depends on how many cores the building machine has (one source gave
+# k_bicgstab 127 or 64 registers and k_wpcg 156 or 124; the 512 x 1024 pressure solve took 233 or 251 ms and other bits).
+FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "--fmad=false", "-std=c++17",
          "-Xcompiler", "-fPIC", "-shared", "-I" + os.path.join(ROOT, "include")]
 
 
