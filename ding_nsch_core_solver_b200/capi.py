@@ -31,6 +31,8 @@ STATUS = {0: "ok", 1: "invalid argument", 2: "invalid configuration", 3: "CUDA e
           6: "pcg breakdown", 7: "bicgstab breakdown", 8: "device wait timed out",
           9: "non-finite diagnostic detected", 10: "unsupported configuration"}
 
+SOLVER_FORM = ("none", "sweep_order", "staged_wavefront", "wavefront", "level_ring", "lines", "level_loop")
+
 
 class BC(C.Structure):
     _fields_ = [("type", C.c_int), ("value", C.c_double)]
@@ -148,6 +150,7 @@ def load():
         "dn_last_phase_times": (I, [H, DP]),
         "dn_kernel_launches": (C.c_longlong, [H]),
         "dn_profile_counters": (I, [H, DP, I]),
+        "dn_solver_forms": (I, [H, C.POINTER(I), C.POINTER(I)]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)
@@ -376,6 +379,12 @@ class Solver:
         out = (C.c_double * count)()
         self._check(self._lib.dn_profile_counters(self._h, out, count))
         return list(out)
+
+    def solver_forms(self) -> dict:
+        """The kernel forms of the CH and pressure PCG solves (dn_solver_forms), by name."""
+        ch, p = C.c_int(), C.c_int()
+        self._check(self._lib.dn_solver_forms(self._h, C.byref(ch), C.byref(p)))
+        return {"ch": SOLVER_FORM[ch.value], "pressure": SOLVER_FORM[p.value]}
 
     def kernel_launches(self) -> int:
         return int(self._lib.dn_kernel_launches(self._h))

@@ -593,6 +593,7 @@ struct dn_handle {
   int sw5_blocks_by_sw[kSweepWarpsPerCta + 1] = {};  // the same for each sweep-warp count up to sw5_budget
   size_t sw5_warp_smem[2] = {0, 0};  // per sweep warp, [constant operator, variable operator]
   int smem_optin = 0;
+  size_t device_bytes = 0;  // the device's memory
   // pressure PCG in sweep order (dn_wpcg.cuh): the FP64 form, or the FP32 inner solves of the mixed form.
   // sw = 0: not set up (no memory to spare, or a line too long for the shared hand-over lines)
   struct WPlan {
@@ -718,6 +719,28 @@ dn_status dalloc(dn_handle *h, T **p, size_t count) {
   h->allocations.push_back(q);
   *p = static_cast<T *>(q);
   return DN_OK;
+}
+
+// Buffers of a kernel form that a handle can do without: bounded by the device and the share that the caller declares,
+// never by what happens to be free, so that one configuration takes one path.  False: over the bound, or not to be
+// had (nothing is left behind, no error pending).
+template <typename T>
+bool dalloc_optional(dn_handle *h, T **p, size_t count) {
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  if (bytes > h->device_bytes / 16 / (size_t)std::max(1, h->cfg.device_share)) return false;
+  void *q = nullptr;
+  if (cudaMalloc(&q, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (cudaMemsetAsync(q, 0, bytes, h->stream) != cudaSuccess) {
+    cudaFree(q);
+    cudaGetLastError();
+    return false;
+  }
+  h->allocations.push_back(q);
+  *p = static_cast<T *>(q);
+  return true;
 }
 
 dn_status falloc(dn_handle *h, Fv &f, int nx, int ny, double init) {
@@ -861,6 +884,11 @@ dn_status dev_status_to_dn(dn_handle *h, int st) {
   }
 }
 
+// periodic y: a line's buffers of the 13-point sweeps fit in shared memory
+bool seq13_fits(const Grid &G) {
+  return G.py && (size_t)seq13_smem_doubles_per_row() * G.ny * sizeof(double) <= kSeqSmemMax;
+}
+
 // ---- persistent PCG launch
 // The arguments and launch shape of the persistent PCG kernel k_pcg<S, SWEEP> (and of k_prec_apply, which
 // runs its sweeps alone).
@@ -900,8 +928,7 @@ dn_status pcg_launch_args(dn_handle *h, const double *a, const double *l, const 
   if (S == 13 && SWEEP == 1 && h->rows13.lval != nullptr) {  // ring of kLvlRing levels x nx doubles
     P.rows13 = h->rows13;
     dyn_smem = (size_t)kLvlRing * h->G.nx * sizeof(double);
-  } else if (S == 13 && SWEEP == 1 && h->G.py &&
-             (size_t)seq13_smem_doubles_per_row() * h->G.ny * sizeof(double) <= kSeqSmemMax) {
+  } else if (S == 13 && SWEEP == 1 && seq13_fits(h->G)) {
     P.seq_lines = 1;  // periodic y: line-staged sequential sweeps
     dyn_smem = (size_t)seq13_smem_doubles_per_row() * h->G.ny * sizeof(double);
   }
@@ -1086,8 +1113,8 @@ void wpcg_problem(WArgs<T> &P, const Grid &G, bool var, int prec, int project, i
   P.scale = var ? (T)1 : -P.cy;
 }
 
-// The handle's plan: its buffers only while they take a small part of the free memory (the layout pads short
-// lines), so that a grid that filled the device before still fits.
+// The handle's plan.  Its vectors are beside those on compact rows (76 bytes a cell and the short lines' padding, 124
+// with the variable operator), so they are optional: without them the wavefronts solve.
 template <typename T>
 dn_status wpcg_setup(dn_handle *h) {
   const dn_config &c = h->cfg;
@@ -1107,13 +1134,9 @@ dn_status wpcg_setup(dn_handle *h) {
     W.blocks_by_sw[w] = std::min(kMaxBlocks, occ * h->num_sms);
   }
   if (wpcg_blocks(h->n, h->rows_per_cta, h->cta_cap, w_blocks(c.nx), sw, W.blocks_by_sw[sw]) == 0) return DN_OK;
-  const size_t bytes = wpcg_layout<T>(c.nx, c.ny, px, var, nullptr, nullptr);
-  size_t free_b = 0, total_b = 0;
-  DN_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
-  if (bytes > free_b / 8) return DN_OK;
   char *mem = nullptr;
-  DN_TRY(dalloc(h, &mem, bytes));
-  DN_TRY(dalloc(h, &W.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot));
+  if (!dalloc_optional(h, &W.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot)) return DN_OK;
+  if (!dalloc_optional(h, &mem, wpcg_layout<T>(c.nx, c.ny, px, var, nullptr, nullptr))) return DN_OK;
   W.mem = mem;
   W.sw = sw;
   return DN_OK;
@@ -1200,13 +1223,10 @@ dn_status wch_setup(dn_handle *h) {
   if (nblk > limit) return DN_OK;
   const size_t vp = c_vec_pairs(c.nx, c.ny), line = (size_t)c_line(c.ny), np = (size_t)w_pairs(c.ny);
   const size_t pairs = 13 * vp + 4 * (size_t)nblk * line + (c.periodic_x ? 4 * line + 10 * np : 0);
-  size_t free_b = 0, total_b = 0;
-  DN_CUDA(h, cudaMemGetInfo(&free_b, &total_b));
-  if (pairs * sizeof(Pair<double>) > free_b / 8) return DN_OK;
   Pair<double> *m = nullptr;
-  DN_TRY(dalloc(h, &m, pairs));
   CArgs &A = W.args;
-  DN_TRY(dalloc(h, &A.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot));
+  if (!dalloc_optional(h, &A.slots, (size_t)kMaxBlocks * kWSlotSets * kWSlot)) return DN_OK;
+  if (!dalloc_optional(h, &m, pairs)) return DN_OK;
   auto take = [&](size_t k) {
     Pair<double> *q = m;
     m += k;
@@ -3426,6 +3446,7 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, device);
   h->num_sms = prop.multiProcessorCount;
+  h->device_bytes = prop.totalGlobalMem;
   h->cta_cap = std::max(1, h->num_sms / std::max(1, cfg->device_share));
   h->rows_per_cta = cfg->pcg_rows_per_cta > 0 ? cfg->pcg_rows_per_cta : kPcgRowsPerCta;
   h->mg_cluster_cells = cfg->mg_cluster_cells > 0 ? cfg->mg_cluster_cells : kMgClusterCells;
@@ -3640,10 +3661,9 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
   }
   h->max_coop_blocks = std::min(kMaxBlocks, std::max(1, occ) * h->num_sms);
   if (c.precision != DN_PRECISION_MIXED && solve_ch(c)) A(wch_setup(h));
-  if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG) {
+  if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG)
     A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
-    if (s != DN_OK) return bad(s, "device allocation failed: " + h->err);
-  }
+  if (s != DN_OK) return bad(s, "solver setup failed: " + h->err);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bad(DN_ERR_CUDA, "initial synchronisation failed");
   *out = h;
   return DN_OK;
@@ -4791,6 +4811,22 @@ dn_status dn_last_phase_times(dn_handle *h, double *out) {
 }
 
 long long dn_kernel_launches(const dn_handle *h) { return h ? h->launches : 0; }
+
+dn_status dn_solver_forms(const dn_handle *h, dn_solver_form *ch, dn_solver_form *pressure) {
+  if (!h) return DN_ERR_INVALID_ARGUMENT;
+  if (ch)
+    *ch = h->cp.blocks > 0                ? DN_FORM_SWEEP_ORDER
+          : h->rows13.lval != nullptr     ? DN_FORM_LEVEL_RING
+          : seq13_fits(h->G)              ? DN_FORM_LINES
+                                          : DN_FORM_LEVEL_LOOP;
+  const dn_config &c = h->cfg;
+  if (pressure)
+    *pressure = c.pressure_scheme == DN_P_JACOBI || c.pressure_scheme == DN_P_SPLIT_DCDM_ICPCG ? DN_FORM_NONE
+                : h->wp.sw > 0                                          ? DN_FORM_SWEEP_ORDER
+                : c.precision != DN_PRECISION_MIXED && h->sw5 > 0       ? DN_FORM_STAGED_WAVEFRONT
+                                                                        : DN_FORM_WAVEFRONT;
+  return DN_OK;
+}
 
 dn_status dn_profile_counters(dn_handle *h, double *out, int count) {
   if (!h || !out || count < 0 || count > 64) return DN_ERR_INVALID_ARGUMENT;

@@ -395,6 +395,20 @@ dn_status dn_last_phase_times(dn_handle *h, double *out);
  * [4k] forward sweep, [4k+1] waits for the neighbouring warp, [4k+2] waits for staged inputs,
  * [4k+3] backward sweep; the sweep-order kernel writes [4k] and [4k+3] of its blocks.  `count` <= 64. */
 dn_status dn_profile_counters(dn_handle *h, double *out, int count);
+/* Which form of the preconditioner's sweeps the handle's incomplete-factor PCG solves run (either may be NULL), chosen at
+ * dn_create from the grid, the boundary, the scheme, device_share and the device's size: `ch` of the FP64
+ * Cahn-Hilliard solve, `pressure` of the pressure solve (mixed precision: of its IC inner solver).  A handle whose
+ * optional buffers could not be allocated falls back and says so here. */
+typedef enum {
+  DN_FORM_NONE = 0,             /* the scheme has no such solve */
+  DN_FORM_SWEEP_ORDER = 1,      /* many CTAs, vectors in sweep order */
+  DN_FORM_STAGED_WAVEFRONT = 2, /* pressure: rows staged in shared memory */
+  DN_FORM_WAVEFRONT = 3,        /* pressure: on global memory */
+  DN_FORM_LEVEL_RING = 4,       /* CH: one CTA, the last levels in shared memory */
+  DN_FORM_LINES = 5,            /* CH, periodic y: one CTA, a line's chain in registers */
+  DN_FORM_LEVEL_LOOP = 6        /* CH: one CTA on global memory */
+} dn_solver_form;
+dn_status dn_solver_forms(const dn_handle *h, dn_solver_form *ch, dn_solver_form *pressure);
 /* Number of this library's kernels launched since the handle was created. */
 long long dn_kernel_launches(const dn_handle *h);
 
