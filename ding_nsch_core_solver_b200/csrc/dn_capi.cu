@@ -1064,7 +1064,9 @@ const void *wpcg_kernel(bool var, bool px, bool py) {
 
 // Sweep warps (blocks) per CTA: one.  Two on an SM slow each other down by more than the shorter hand-over inside a
 // CTA saves (192 x 384 split: 59.5 us of sweeps per iteration with one, 61.0 with two; 512 x 1024: 152 and 161); more
-// only where the CTAs would not fit the caller's share otherwise.
+// only where the CTAs would not fit the caller's share otherwise.  0 where they do not fit it at all: one CTA takes an
+// SM, and instances side by side with more CTAs than SMs would wait for one another's, up to the time limit (the
+// wavefronts put up to four sweep warps in a CTA).
 template <typename T>
 int wpcg_sweep_warps(int nx, int ny, bool px, bool py, bool var, int optin, int cta_cap, int asked, size_t *warp_smem,
                      int *budget) {
@@ -1082,7 +1084,7 @@ int wpcg_sweep_warps(int nx, int ny, bool px, bool py, bool var, int optin, int 
   if (asked > 0) return std::min(asked, most);
   int sw = 1;
   while (sw < most && (nblk + sw - 1) / sw > cta_cap) ++sw;
-  return sw;
+  return (nblk + sw - 1) / sw > cta_cap ? 0 : sw;
 }
 
 // CTAs of a solve: about rows_per_cta cells each, within the share and the co-resident limit; 0: not launchable
@@ -1220,7 +1222,8 @@ dn_status wch_setup(dn_handle *h) {
   int occ = 0;
   DN_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_wch, kBlock, c_smem()));
   const int limit = std::min(kMaxBlocks, occ * h->num_sms), nblk = w_blocks(c.nx);
-  if (nblk > limit) return DN_OK;
+  // a block is a CTA, which takes an SM (c_smem): within the caller's share, or the one-CTA forms
+  if (nblk > std::min(limit, h->cta_cap)) return DN_OK;
   const size_t vp = c_vec_pairs(c.nx, c.ny), line = (size_t)c_line(c.ny), np = (size_t)w_pairs(c.ny);
   const size_t pairs = 13 * vp + 4 * (size_t)nblk * line + (c.periodic_x ? 4 * line + 10 * np : 0);
   Pair<double> *m = nullptr;
@@ -4003,7 +4006,7 @@ dn_status dn_autotune_pressure(dn_handle *h, int *rows_per_cta, int *sweep_warps
   std::vector<int> sws;
   if (fp64 && h->wp.sw > 0) {
     for (int w = 1; w <= h->wp.sw_budget; ++w)
-      if ((w_blocks(h->G.nx) + w - 1) / w <= h->wp.blocks_by_sw[w]) sws.push_back(w);
+      if ((w_blocks(h->G.nx) + w - 1) / w <= std::min(h->cta_cap, h->wp.blocks_by_sw[w])) sws.push_back(w);
   } else if (fp64 && h->sw5 > 0) {
     for (int w = 1; w <= h->sw5_budget; ++w)
       if ((h->nsweep5 + w - 1) / w <= h->sw5_blocks_by_sw[w]) sws.push_back(w);

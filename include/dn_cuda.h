@@ -82,7 +82,8 @@ typedef struct {
   double mixed_inner_tolerance;    /* relative tolerance of each FP32 inner solve (mixed form) */
   int device_share;                /* handles meant to run concurrently on one device (dn_step_batch): each
                                       persistent launch takes at most 1/device_share of the SMs, never fewer
-                                      CTAs than its wavefront needs; 1 = the whole device */
+                                      CTAs than its wavefront needs; 1 = the whole device.  The forms in sweep
+                                      order (dn_solver_forms), a CTA per 32 lines, are taken where they fit it */
   int dcdm_direction_mode;         /* split_dcdm_icpcg directions: 0 icc_preconditioned, 1 identity (config.hpp:51) */
   int dcdm_history_size, dcdm_max_stored_directions, dcdm_restart_interval; /* config.hpp:72-74 */
   int pcg_rows_per_cta;            /* launch shape of the pressure PCG: rows per CTA of its SpMV / update
