@@ -3508,23 +3508,6 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
   A(dalloc(h, &h->l5, 5 * h->n));
   A(dalloc(h, &h->a13, 13 * h->n));
   A(dalloc(h, &h->l13, 13 * h->n));
-  // ordered factor rows for the ring-based CH sweeps: neither direction periodic and the ring fits in shared
-  // memory (periodic x keeps the level sweep on global memory: a self-checked run of the wrapped rows found
-  // no bad index, but the unchecked build faulted on them, so that combination stays off)
-  if (!c.periodic_x && !c.periodic_y && (size_t)kLvlRing * nx * sizeof(double) <= 96 * 1024 && nx < 65536) {
-    const int k = 6;
-    h->rows13.k = k;
-    A(dalloc(h, &h->rows13.lval, (size_t)k * h->n));
-    A(dalloc(h, &h->rows13.uval, (size_t)k * h->n));
-    A(dalloc(h, &h->rows13.lcol, (size_t)k * h->n));
-    A(dalloc(h, &h->rows13.ucol, (size_t)k * h->n));
-    A(dalloc(h, &h->rows13.lsrc, (size_t)k * h->n));
-    A(dalloc(h, &h->rows13.usrc, (size_t)k * h->n));
-  }
-  // the CH PCG kernel's dynamic shared memory (the ring, or the periodic-y line buffers): allow the largest
-  // amount any handle uses
-  if ((h->rows13.lval != nullptr || c.periodic_y) && s == DN_OK)
-    cudaFuncSetAttribute(k_pcg<13, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmemMax);
   h->ml = MomLayout{nx, ny, c.periodic_x, c.periodic_y, (long long)(nx + 1) * ny, (long long)nx * (ny + 1)};
   h->nm = h->ml.nu + h->ml.nv;
   if (h->nm >= (1LL << 31))
@@ -3664,6 +3647,24 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
   }
   h->max_coop_blocks = std::min(kMaxBlocks, std::max(1, occ) * h->num_sms);
   if (c.precision != DN_PRECISION_MIXED && solve_ch(c)) A(wch_setup(h));
+  // ordered factor rows (192 bytes a cell) for the ring-based CH sweeps, where the sweep-order PCG is not set up:
+  // neither direction periodic and the ring fits in shared memory (periodic x then takes the level sweep on global
+  // memory: a self-checked run of the wrapped rows found no bad index, but the unchecked build faulted on them, so
+  // that combination stays off)
+  if (h->cp.blocks == 0 && !c.periodic_x && !c.periodic_y && (size_t)kLvlRing * nx * sizeof(double) <= 96 * 1024 && nx < 65536) {
+    const int k = 6;
+    h->rows13.k = k;
+    A(dalloc(h, &h->rows13.lval, (size_t)k * h->n));
+    A(dalloc(h, &h->rows13.uval, (size_t)k * h->n));
+    A(dalloc(h, &h->rows13.lcol, (size_t)k * h->n));
+    A(dalloc(h, &h->rows13.ucol, (size_t)k * h->n));
+    A(dalloc(h, &h->rows13.lsrc, (size_t)k * h->n));
+    A(dalloc(h, &h->rows13.usrc, (size_t)k * h->n));
+  }
+  // the CH PCG kernel's dynamic shared memory (the ring, or the periodic-y line buffers): allow the largest
+  // amount any handle uses
+  if ((h->rows13.lval != nullptr || c.periodic_y) && s == DN_OK)
+    cudaFuncSetAttribute(k_pcg<13, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmemMax);
   if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG)
     A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
   if (s != DN_OK) return bad(s, "solver setup failed: " + h->err);

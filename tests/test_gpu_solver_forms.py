@@ -64,15 +64,33 @@ def measure(spare):
     return dict(first=first, then=then, c=rel_l2(c1, c), p=rel_l2(p1, p), held=len(held))
 
 
+def footprint(periodic_x):
+    import ding_nsch_core_solver_b200 as dn
+    from test_gpu_parity import unit
+
+    cfg = unit(**dict(GRID, periodic_x=periodic_x))
+    dn.Solver(cfg).close()
+    before = free_bytes()
+    s = dn.Solver(cfg)
+    used = before - free_bytes()
+    forms = s.solver_forms()
+    s.close()
+    return dict(forms, bytes=used)
+
+
+def child(*args):
+    """This file as a program; its last line."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here, os.environ.get("PYTHONPATH", "")]))
+    run = subprocess.run([sys.executable, os.path.abspath(__file__), *args], capture_output=True, text=True, env=env, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+    return json.loads(run.stdout.splitlines()[-1])
+
+
 @pytest.mark.parametrize("spare", [1.0, -0.5], ids=["room", "no room"])
 def test_forms_do_not_follow_the_free_memory(spare):
     """room: the handle fits with as much again as its optional buffers to spare.  no room: half of them is missing."""
-    here = os.path.dirname(os.path.abspath(__file__))
-    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here, os.environ.get("PYTHONPATH", "")]))
-    run = subprocess.run([sys.executable, os.path.abspath(__file__), str(spare)], capture_output=True, text=True, env=env,
-                         timeout=300)
-    assert run.returncode == 0, run.stderr[-2000:]
-    got = json.loads(run.stdout.splitlines()[-1])
+    got = child("free", str(spare))
     assert got["first"] == {"ch": "sweep_order", "pressure": "sweep_order"}
     if spare > 0:
         assert got["then"] == got["first"]
@@ -83,5 +101,13 @@ def test_forms_do_not_follow_the_free_memory(spare):
     assert got["c"] <= 1e-5 and got["p"] <= 2e-2
 
 
+def test_a_handle_holds_no_rows_of_a_form_that_it_does_not_run():
+    """The ordered factor rows of the level ring (192 bytes a cell) belong to walled boxes that run it; a box swept by
+    many CTAs takes what its periodic-x twin takes, which has its wrap lines on top (8 MiB for the allocator's steps)."""
+    walls, channel = child("rows", "0"), child("rows", "1")
+    assert walls["ch"] == channel["ch"] == "sweep_order"
+    assert walls["bytes"] <= channel["bytes"] + (8 << 20)
+
+
 if __name__ == "__main__":
-    print(json.dumps(measure(float(sys.argv[1]))))
+    print(json.dumps(measure(float(sys.argv[2])) if sys.argv[1] == "free" else footprint(sys.argv[2] == "1")))
