@@ -922,14 +922,12 @@ dn_status pcg_launch_args(dn_handle *h, const double *a, const double *l, const 
   P.warp_smem = 0;
   P.rows13 = Rows13{};
   size_t dyn_smem = 0;
-  P.seq_lines = 0;
   P.mon = S == 5 ? h->mon : nullptr;
   P.mon_cap = S == 5 ? h->mon_cap : 0;
   if (S == 13 && SWEEP == 1 && h->rows13.lval != nullptr) {  // ring of kLvlRing levels x nx doubles
     P.rows13 = h->rows13;
     dyn_smem = (size_t)kLvlRing * h->G.nx * sizeof(double);
-  } else if (S == 13 && SWEEP == 1 && seq13_fits(h->G)) {
-    P.seq_lines = 1;  // periodic y: line-staged sequential sweeps
+  } else if (SWEEP == 5) {
     dyn_smem = (size_t)seq13_smem_doubles_per_row() * h->G.ny * sizeof(double);
   }
   // about 512 rows per CTA: the SpMV / update phases are latency-bound, so more CTAs shorten them
@@ -2177,6 +2175,9 @@ dn_status ensure_ch_system(dn_handle *h, double alpha0) {
 // The ILDLT-preconditioned CG: swept by many CTAs, or (periodic y) by one.
 dn_status run_ch_ldlt(dn_handle *h, double out[4], double *rec) {
   if (h->cp.blocks > 0) return run_wch(h, out, rec);
+  if (seq13_fits(h->G))
+    return run_pcg<13, 5>(h, h->a13, h->l13, h->dinv13, kPrecLDLT, 0, h->cfg.ch_inner_iterations, h->cfg.ch_tolerance, out,
+                          rec);
   return run_pcg<13, 1>(h, h->a13, h->l13, h->dinv13, kPrecLDLT, 0, h->cfg.ch_inner_iterations, h->cfg.ch_tolerance, out,
                         rec);
 }
@@ -3636,6 +3637,9 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg<5, 0>, kBlock, 0);
   int occ2 = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_pcg<13, 1>, kBlock, 0);
+  int occ5 = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ5, k_pcg<13, 5>, kBlock, 0);
+  occ2 = std::min(occ2, occ5);
   int occ3 = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_bicgstab, kBlock, 0);
   h->bicg_occ = std::max(1, occ3);
@@ -3661,10 +3665,11 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
     A(dalloc(h, &h->rows13.lsrc, (size_t)k * h->n));
     A(dalloc(h, &h->rows13.usrc, (size_t)k * h->n));
   }
-  // the CH PCG kernel's dynamic shared memory (the ring, or the periodic-y line buffers): allow the largest
+  // the one-CTA CH PCG kernels' dynamic shared memory (the ring, the periodic-y line buffers): allow the largest
   // amount any handle uses
   if ((h->rows13.lval != nullptr || c.periodic_y) && s == DN_OK)
-    cudaFuncSetAttribute(k_pcg<13, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmemMax);
+    for (const void *k : {(const void *)k_pcg<13, 1>, (const void *)k_pcg<13, 5>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmemMax);
   if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG)
     A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
   if (s != DN_OK) return bad(s, "solver setup failed: " + h->err);
@@ -4964,6 +4969,8 @@ dn_status static_setup(int device, StaticDevice *out, char *err, size_t err_len)
     int occ = 0, occ2 = 0, occ3 = 0;
     DN_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg<5, 0>, kBlock, 0));
     DN_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_pcg<13, 1>, kBlock, 0));
+    DN_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_pcg<13, 5>, kBlock, 0));
+    occ2 = std::min(occ2, occ3);
     DN_SCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_bicgstab, kBlock, 0));
     occ = std::min(occ, std::min(occ2, occ3));
     t.max_coop_blocks = std::min(kMaxBlocks, std::max(1, occ) * t.num_sms);

@@ -469,7 +469,6 @@ struct PcgArgsT {
   Rows13 rows13;   // ordered factor rows of the 13-point operator (SWEEP 1, y not periodic); lval null: unused
   Sweep5T<T> s5;   // staged wavefront (SWEEP 3)
   int warp_smem;   // shared-memory bytes per sweep warp (SWEEP 3)
-  int seq_lines;   // 13-point with periodic y: 1 = line-staged sequential sweeps (seq13 dynamic smem)
   double *mon;     // per-iteration record [iteration][4]: abs residual, rel residual, iterate residual, alpha
   int mon_cap;     // iterations the record holds (0: no record)
 };
@@ -1001,7 +1000,9 @@ __device__ void apply_seq13(const PcgArgs &P, double m_r, double (&acc)[3], doub
 
 // One persistent launch runs the whole PCG.  SWEEP: 0 = 5-point pipelined wavefront on global memory,
 // 1 = level-scheduled slot factor (CTA 0), 2 = diagonal, 3 = 5-point wavefront staged through shared memory,
-// 4 = the staged wavefront with the periodic-x wrap terms (nx >= 32).
+// 4 = the staged wavefront with the periodic-x wrap terms (nx >= 32), 5 = 13-point factor with periodic y, line by
+// line (CTA 0; apply_seq13).  5 is a kernel of its own: as a branch of 1 it made the level ring spill registers
+// (Cahn-Hilliard solve at 192 x 384 9.1 -> 12.5 ms).
 // The residual r is kept unprojected in memory; the mean of the latest update (m_r) is subtracted on the
 // fly by the preconditioner and folded in by the next update, which equals projecting r after every
 // update (pressure.cpp:225-239 applied in ch_sparse_krylov.hpp:602-605).
@@ -1197,12 +1198,17 @@ __global__ void __launch_bounds__(kBlock) k_pcg(PcgArgsT<T> P) {
         if (blockIdx.x == 0) {
           if (S == 13 && P.rows13.lval != nullptr && P.rows13.k == 6)
             apply_levels13_ring<6>(P, m_r_now, acc, (double *)dsm);
-          else if (S == 13 && P.seq_lines && P.prec == kPrecICC)
-            apply_seq13<true>(P, m_r_now, acc, (double *)dsm);
-          else if (S == 13 && P.seq_lines)
-            apply_seq13<false>(P, m_r_now, acc, (double *)dsm);
           else
             apply_levels<S>(P, m_r_now, acc);
+        }
+      }
+    } else if (SWEEP == 5) {
+      if constexpr (S == 13 && sizeof(T) == sizeof(double)) {
+        if (blockIdx.x == 0) {
+          if (P.prec == kPrecICC)
+            apply_seq13<true>(P, m_r_now, acc, (double *)dsm);
+          else
+            apply_seq13<false>(P, m_r_now, acc, (double *)dsm);
         }
       }
     } else {
