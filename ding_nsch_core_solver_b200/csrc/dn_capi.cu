@@ -594,6 +594,9 @@ struct dn_handle {
   size_t sw5_warp_smem[2] = {0, 0};  // per sweep warp, [constant operator, variable operator]
   int smem_optin = 0;
   size_t device_bytes = 0;  // the device's memory
+  // the staged wavefront in FP32: the mixed form's IC inner solver where the sweep order does not take the grid
+  int sw5f = 0, sw5f_blocks_max = 0;
+  size_t sw5f_warp_smem = 0;
   // pressure PCG in sweep order (dn_wpcg.cuh): the FP64 form, or the FP32 inner solves of the mixed form.
   // sw = 0: not set up (no memory to spare, or a line too long for the shared hand-over lines)
   struct WPlan {
@@ -889,6 +892,41 @@ bool seq13_fits(const Grid &G) {
   return G.py && (size_t)seq13_smem_doubles_per_row() * G.ny * sizeof(double) <= kSeqSmemMax;
 }
 
+// The staged wavefront's arguments; the hand-over lines are FP64's, which FP32 uses half of.
+template <typename T>
+Sweep5T<T> sweep5_args(dn_handle *h, const T *a, const T *dinv, int prec, T *r, T *y, T *z, int sw, int warp_smem) {
+  Sweep5T<T> W{};
+  W.nx = h->G.nx;
+  W.ny = h->G.ny;
+  W.n = (int)h->n;
+  W.px = h->G.px;
+  W.py = h->G.py;
+  W.prec = prec;
+  W.varcoef = use_split(h->cfg) ? 0 : 1;
+  W.aW = a;
+  W.aS = a + h->n;
+  W.aN = a + 3 * h->n;
+  W.aE = a + 4 * h->n;
+  W.cx = (T)(-(1.0 / (h->G.dx * h->G.dx)));
+  W.cy = (T)(-(1.0 / (h->G.dy * h->G.dy)));
+  W.dinv = dinv;
+  W.r = r;
+  W.y = y;
+  W.z = z;
+  W.bnd_f = reinterpret_cast<T *>(h->bnd_f);
+  W.bnd_b = reinterpret_cast<T *>(h->bnd_b);
+  W.wline0 = reinterpret_cast<T *>(h->wline0);
+  W.zlast = reinterpret_cast<T *>(h->zlast);
+  W.prog_f = h->prog;
+  W.prog_b = h->prog + kMaxBlocks * 8;
+  W.nsweep = h->nsweep5;
+  W.sw = sw;
+  W.status = h->status;
+  W.warp_smem = warp_smem;
+  W.prof = h->prof;
+  return W;
+}
+
 // ---- persistent PCG launch
 // The arguments and launch shape of the persistent PCG kernel k_pcg<S, SWEEP> (and of k_prec_apply, which
 // runs its sweeps alone).
@@ -937,38 +975,9 @@ dn_status pcg_launch_args(dn_handle *h, const double *a, const double *l, const 
   blocks = std::max(blocks, (h->nsweep + kBlock / 32 - 1) / (kBlock / 32));  // the wavefront warps' CTAs
   blocks = std::max(1, std::min(blocks, h->max_coop_blocks));
   if (SWEEP == 3 || SWEEP == 4) {
-    const dn_config &c = h->cfg;
-    const bool var = !use_split(c);
-    Sweep5 &W = P.s5;
-    W.nx = h->G.nx;
-    W.ny = h->G.ny;
-    W.n = (int)h->n;
-    W.px = h->G.px;
-    W.py = h->G.py;
-    W.prec = prec;
-    W.varcoef = var ? 1 : 0;
-    W.aW = a;
-    W.aS = a + h->n;
-    W.aN = a + 3 * h->n;
-    W.aE = a + 4 * h->n;
-    W.cx = -(1.0 / (h->G.dx * h->G.dx));
-    W.cy = -(1.0 / (h->G.dy * h->G.dy));
-    W.dinv = dinv;
-    W.r = h->r;
-    W.y = h->y;
-    W.z = h->z;
-    W.bnd_f = h->bnd_f;
-    W.bnd_b = h->bnd_b;
-    W.wline0 = h->wline0;
-    W.zlast = h->zlast;
-    W.prog_f = h->prog;
-    W.prog_b = h->prog + kMaxBlocks * 8;
-    W.nsweep = h->nsweep5;
-    W.sw = h->sw5;
-    W.status = h->status;
+    const bool var = !use_split(h->cfg);
     P.warp_smem = (int)h->sw5_warp_smem[var ? 1 : 0];
-    W.warp_smem = P.warp_smem;
-    W.prof = h->prof;
+    P.s5 = sweep5_args<double>(h, a, dinv, prec, h->r, h->y, h->z, h->sw5, P.warp_smem);
     dyn_smem = 64 + (size_t)h->sw5 * P.warp_smem;
     const int sweep_ctas = (h->nsweep5 + h->sw5 - 1) / h->sw5;
     blocks = std::max(blocks, sweep_ctas);
@@ -1293,6 +1302,33 @@ dn_status run_pcg(dn_handle *h, const double *a, const double *l, const double *
   return pcg_launch(h, (const void *)k_pcg<S, SWEEP>, blocks, kBlock, args, dyn_smem, S == 5 ? 4 : 5, out, rec);
 }
 
+const void *staged32_kernel(bool px) {
+  return px ? (const void *)k_pcg<5, 4, float> : (const void *)k_pcg<5, 3, float>;
+}
+
+// The FP32 staged wavefront's sweep warps per CTA, where rows fit in shared memory and (periodic x) line nx-1 lies in
+// another warp than line 0.  Without it a grid such as 256 x 32 with periodic y, whose lines are too short for the sweep
+// order, ran the wavefront on global memory: 28 -> 470 ms of pressure solve.
+void staged32_setup(dn_handle *h) {
+  const dn_config &c = h->cfg;
+  const bool px = c.periodic_x != 0;
+  if (px && h->nsweep5 < 2) return;
+  const void *kern = staged32_kernel(px);
+  const size_t per = (sweep_warp_smem(use_split(c) ? 2 : 4, c.ny, 4, px) + 15) & ~(size_t)15;
+  cudaFuncAttributes fa{};
+  cudaFuncGetAttributes(&fa, kern);
+  const size_t used = 64 + fa.sharedSizeBytes, budget = (size_t)h->smem_optin > used ? (size_t)h->smem_optin - used : 0;
+  int sw = std::min((int)std::min<size_t>(kSweepWarpsPerCta, budget / per), h->nsweep5);
+  if (sw > 0 && c.sweep_warps_per_cta > 0) sw = std::min(sw, c.sweep_warps_per_cta);
+  if (sw == 0) return;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, h->smem_optin - (int)fa.sharedSizeBytes);
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBlock, 64 + (size_t)sw * per);
+  h->sw5f_warp_smem = per;
+  h->sw5f_blocks_max = std::min(kMaxBlocks, std::max(0, occ) * h->num_sms);
+  h->sw5f = h->sw5f_blocks_max > 0 ? sw : 0;
+}
+
 // One FP32 inner PCG solve (the persistent kernels instantiated for float) on the handle's FP32 buffers, from a
 // zero iterate.
 dn_status run_pcg32(dn_handle *h, int prec, int project, int max_it, double tol, double out[4]) {
@@ -1336,11 +1372,22 @@ dn_status run_pcg32(dn_handle *h, int prec, int project, int max_it, double tol,
                                         std::max<long long>(h->nsweep, (h->n + rows_per_cta - 1) / rows_per_cta));
   blocks = std::max(blocks, (h->nsweep + kBlock / 32 - 1) / (kBlock / 32));  // the wavefront warps' CTAs
   blocks = std::max(1, std::min(blocks, h->max_coop_blocks));
-  if ((long long)blocks * (kBlock / 32) < h->nsweep)
+  const void *kern = (const void *)k_pcg<5, 0, float>;
+  size_t dyn_smem = 0;
+  if (h->sw5f > 0) {
+    kern = staged32_kernel(h->G.px != 0);
+    P.warp_smem = (int)h->sw5f_warp_smem;
+    P.s5 = sweep5_args<float>(h, h->fa5, h->fdinv5, prec, h->fr, h->fy, h->fz, h->sw5f, P.warp_smem);
+    dyn_smem = 64 + (size_t)h->sw5f * P.warp_smem;
+    const int sweep_ctas = (h->nsweep5 + h->sw5f - 1) / h->sw5f;
+    blocks = std::min(std::max(blocks, sweep_ctas), h->sw5f_blocks_max);
+    if (blocks < sweep_ctas) return fail(h, DN_ERR_UNSUPPORTED, "not enough co-resident CTAs for the wavefront");
+  } else if ((long long)blocks * (kBlock / 32) < h->nsweep) {
     return fail(h, DN_ERR_UNSUPPORTED, "grid too wide for the co-resident wavefront warps");
+  }
   DN_TRY(reset_sync(h));
   void *args[] = {&P};
-  return pcg_launch(h, (const void *)k_pcg<5, 0, float>, blocks, kBlock, args, 0, 4, out, nullptr);
+  return pcg_launch(h, kern, blocks, kBlock, args, dyn_smem, 4, out, nullptr);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -3672,6 +3719,7 @@ dn_status dn_create(const dn_config *cfg, int device, dn_handle **out) {
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmemMax);
   if (c.pressure_scheme != DN_P_JACOBI && c.pressure_scheme != DN_P_SPLIT_DCDM_ICPCG)
     A(c.precision == DN_PRECISION_MIXED ? wpcg_setup<float>(h) : wpcg_setup<double>(h));
+  if (c.precision == DN_PRECISION_MIXED && h->wp.sw == 0) staged32_setup(h);
   if (s != DN_OK) return bad(s, "solver setup failed: " + h->err);
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bad(DN_ERR_CUDA, "initial synchronisation failed");
   *out = h;
@@ -4831,9 +4879,9 @@ dn_status dn_solver_forms(const dn_handle *h, dn_solver_form *ch, dn_solver_form
   const dn_config &c = h->cfg;
   if (pressure)
     *pressure = c.pressure_scheme == DN_P_JACOBI || c.pressure_scheme == DN_P_SPLIT_DCDM_ICPCG ? DN_FORM_NONE
-                : h->wp.sw > 0                                          ? DN_FORM_SWEEP_ORDER
-                : c.precision != DN_PRECISION_MIXED && h->sw5 > 0       ? DN_FORM_STAGED_WAVEFRONT
-                                                                        : DN_FORM_WAVEFRONT;
+                : h->wp.sw > 0 ? DN_FORM_SWEEP_ORDER
+                : (c.precision == DN_PRECISION_MIXED ? h->sw5f : h->sw5) > 0 ? DN_FORM_STAGED_WAVEFRONT
+                                                                             : DN_FORM_WAVEFRONT;
   return DN_OK;
 }
 
