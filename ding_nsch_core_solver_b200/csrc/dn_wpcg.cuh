@@ -593,6 +593,10 @@ __device__ __forceinline__ bool w_help(const WArgs<T> &P, const WWarp<T> &W, lon
   return told >= S;
 }
 
+// A sum as a slot holds it: a NaN that carries the empty slot's bits (a state filled with 0xff has it) as another NaN,
+// so that the solve breaks down on it, as on any NaN, and does not wait for a value that has come.
+__device__ __forceinline__ double slot_value(double v) { return isnan(v) ? __longlong_as_double(0x7ff8000000000000ll) : v; }
+
 // Sum of K values over the CTA, then over the grid: see the reductions' note at the top.  Every CTA of
 // [0, writers) publishes its sums in its slot of set `set`, empties set `next` (read two reductions ago), and
 // every CTA adds all slots in the same order.  False when a wait gave up (on every thread of the CTA).
@@ -612,7 +616,8 @@ __device__ __forceinline__ bool w_reduce(double (&v)[K], double *slots, int set,
       __threadfence();
 #pragma unroll
       for (int k = 0; k < KP; ++k)
-        st_pair_if((Pair<double> *)(mine + set * kWSlot + 2 * k), Pair<double>{v[2 * k], 2 * k + 1 < K ? v[2 * k + 1] : 0.0}, true);
+        st_pair_if((Pair<double> *)(mine + set * kWSlot + 2 * k),
+                   Pair<double>{slot_value(v[2 * k]), 2 * k + 1 < K ? slot_value(v[2 * k + 1]) : 0.0}, true);
     }
   }
   double u[K];
