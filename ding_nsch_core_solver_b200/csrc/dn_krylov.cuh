@@ -1092,6 +1092,13 @@ __device__ __forceinline__ void pcg_update_rows(const PcgArgsT<T> &P, long long 
   }
 }
 
+// The smallest p.Ap of an iteration: the reference's bound (ch_sparse_krylov.hpp:588-590) in FP64.  An FP32 solve is an inner
+// one, of a residual of any size, so its bound is that of a p of zeros alone.
+template <typename T>
+__device__ constexpr double pcg_pap_min() {
+  return sizeof(T) == sizeof(float) ? 1.0e-300 : 1.0e-30;
+}
+
 template <int S, int SWEEP, typename T = double>
 __global__ void __launch_bounds__(kBlock) k_pcg(PcgArgsT<T> P) {
   __shared__ double sh[8 * 32 + 8];
@@ -1249,7 +1256,7 @@ __global__ void __launch_bounds__(kBlock) k_pcg(PcgArgsT<T> P) {
     if (!grid_sum<3>(v, P.partials, parity, sh, bar)) return;
     const double m_p = P.project ? v[0] / dn_ : 0.0;
     const double pap = P.project ? v[1] - m_p * v[2] : v[1];
-    if (!isfinite(pap) || fabs(pap) < 1.0e-30) {
+    if (!isfinite(pap) || fabs(pap) < pcg_pap_min<T>()) {
       if (threadIdx.x == 0) atomicCAS(P.status, kDevOk, kDevPcgBreakdownPap);
       return;
     }

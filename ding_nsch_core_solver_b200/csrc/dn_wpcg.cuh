@@ -47,6 +47,7 @@
 #include <type_traits>
 
 #include "dn_common.cuh"
+#include "dn_krylov.cuh"
 #include "dn_wavefront.cuh"
 
 namespace dn {
@@ -993,7 +994,8 @@ __global__ void __launch_bounds__(kWBlock, 1) k_wpcg(WArgs<T> P) {
 
   unsigned long long t_p1 = 0, t_p2 = 0, t_pc = 0;
   double m_x = 0.0, rz_old = 0.0;
-  const double scale = (double)P.scale, pap_min = 1.0e-30 * scale * scale;  // z and p carry the factor
+  const double scale = (double)P.scale;  // z and p carry the factor
+  const double pap_min = sizeof(T) == sizeof(float) ? pcg_pap_min<T>() : pcg_pap_min<T>() * scale * scale;
   P2 *p_old = P.p0, *p_new = P.p1;
   const int max_it = P.max_it > 1 ? P.max_it : 1;
   for (int it = 0;; ++it) {

@@ -46,3 +46,19 @@ def test_short_periodic_lines_take_the_staged_wavefront(dn, nx, ny, px, scheme):
     finally:
         plain.close()
         mixed.close()
+
+
+@pytest.mark.parametrize("scheme", ["split_icpcg", "icpcg", "split_ildlt_pcg"])
+@pytest.mark.parametrize("nx,ny,px,py", [(64, 24, 0, 0), (64, 24, 0, 1), (130, 24, 0, 0), (97, 32, 0, 1), (97, 32, 0, 0), (64, 64, 0, 1),
+                                         (64, 64, 0, 0)])
+def test_a_small_right_hand_side_is_no_breakdown(dn, nx, ny, px, py, scheme):
+    """A drop at rest: a small right-hand side, whose later corrections have p.Ap under 1e-30."""
+    cfg = unit(nx=nx, ny=ny, lx=nx / 64.0, ly=ny / 64.0, interface_center_x=nx / 128.0, interface_center_y=ny / 128.0,
+               interface_radius=0.1, periodic_x=bool(px), periodic_y=bool(py), pressure_scheme=scheme, dt=1e-4, density_ratio=10.0)
+    s = dn.Solver(dict(cfg, precision="mixed", mixed_preconditioner="ic"))
+    try:
+        s.initialize()
+        for step in range(2):
+            assert s.step(step)["pressure_residual"] < 1e-10
+    finally:
+        s.close()
